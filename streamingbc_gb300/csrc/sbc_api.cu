@@ -655,7 +655,7 @@ int sbc_graph_create(sbc_graph** out, int64_t nv, const int64_t* off, const int6
         int sm_count = 0;
         cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
         if ((e = sbc::build_adjacency(nv, off, adj, g->d_row, g->d_deg, deg, g->d_col, std::max(sm_count, 1),
-                                      g->stream))) {
+                                      g->stream, &g->edge_skew))) {
             sbc_graph_destroy(g);
             return cuda_fail(e, "sbc_graph_create adjacency build");
         }
@@ -723,6 +723,7 @@ int sbc_graph_insert_directed(sbc_graph* g, int64_t from, int64_t to, int* resul
     CK(cudaMemcpyAsync(&code, g->d_ins + 2 * g->ins_capacity, sizeof code, cudaMemcpyDeviceToHost, g->stream));
     CK(cudaStreamSynchronize(g->stream));
     if (code == -2) return check_graph_err(g);
+    if (code == 1) g->edge_skew += sbc::edge_mix((int)from, (int)to);
     if (result) *result = code < 0 ? -1 : code;
     return SBC_OK;
 }
@@ -932,10 +933,7 @@ int sbc_static_init(sbc_forest* f)
     if (!f) return fail(SBC_ERR_ARG, "sbc_static_init: null");
     if (use_device(f->g->device)) return SBC_ERR_CUDA;
     CK(sbc::launch_static(f));
-    CK(sbc::launch_dist2_rows(f, nullptr, nullptr));
     CK(sbc::launch_l2mask_build_all(f));
-    CK(sbc::launch_level_hist(f));
-    CK(sbc::launch_roster_build(f));
     f->initialized = true;
     return SBC_OK;
 }
@@ -1184,6 +1182,7 @@ int sbc_graph_remove_directed(sbc_graph* g, int64_t from, int64_t to, int* resul
     CK(sbc::launch_remove(g, (int)from, (int)to, true, g->d_err + 1));
     CK(cudaMemcpyAsync(result, g->d_err + 1, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
     CK(cudaStreamSynchronize(g->stream));
+    if (*result == 1) g->edge_skew -= sbc::edge_mix((int)from, (int)to);
     return SBC_OK;
 }
 

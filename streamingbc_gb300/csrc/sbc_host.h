@@ -147,6 +147,7 @@ struct sbc_graph {
     // forests bound to this graph; destroying the graph detaches them
     std::vector<sbc_forest*> forests;
     bool last_directed = false;  // the staged insertions were appended one direction only
+    unsigned long long edge_skew = 0;  // edge_mix summed over the live slots: 0 when every edge has both directions
 
     sbc::DevGraph dev() const
     {
@@ -378,7 +379,6 @@ inline ForestSlot forest_slot(const sbc_forest* f, int n)
     return s;
 }
 
-int static_workers_per_sm();
 int update_variant_count();
 int update_default_variant();
 int update_variant_threads(int v);
@@ -387,10 +387,10 @@ int update_workers_per_sm(int v);
 int report_error(int code, const char* fmt, ...);
 // Scatters the caller's host CSR into the device slack layout (d_row, d_deg
 // already set; deg = the live degrees) and sorts every vertex's list on the
-// device.  Synchronous on s.
+// device; *skew gets the edge skew.  Synchronous on s.
 cudaError_t build_adjacency(int64_t nv, const int64_t* off, const int64_t* adj, const int64_t* d_row,
                             const int32_t* d_deg, const std::vector<int32_t>& deg, int32_t* d_col, int sm_count,
-                            cudaStream_t s);
+                            cudaStream_t s, unsigned long long* skew);
 cudaError_t launch_static(sbc_forest* f);
 // Classify + cull + update for insertions already staged in g->d_ins
 // (u, v, ok rows).  `all_visible` ignores the per-slot sequence numbers.
@@ -418,9 +418,9 @@ cudaError_t launch_delete(sbc_forest* f, int u, int v, const int* d_removed);
 // Every root through the n deletions marked in g's staging (launch_mark_removed),
 // in one persistent launch; dirty roots are left for launch_delete_finish.
 cudaError_t launch_delete_batch(sbc_forest* f, int n);
-// Static recompute of the roots listed (device list and count) or, with a
-// null list, of all roots.
-cudaError_t launch_static_list(sbc_forest* f, const int* d_list, const int* d_nlist);
+// Static recompute of the n roots listed (device list and count) or, with a
+// null list, of all roots: their rows, level histograms and rosters.
+cudaError_t launch_static_list(sbc_forest* f, const int* d_list, const int* d_nlist, int64_t n);
 // Whole-GPU recompute of the listed root rows (rows on the host, d_rows the
 // same list on the device), all of them level by level together
 // (level-synchronous, synchronous); used by deletions on graphs of at least

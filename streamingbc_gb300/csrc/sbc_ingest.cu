@@ -36,16 +36,26 @@
 
 namespace sbc {
 
-// col[row[v] + i] = adj[off[v] + i] for the listed vertices' live neighbours.
+// col[row[v] + i] = adj[off[v] + i] for the listed vertices' live neighbours,
+// and the edge skew of all of them added into *skew.
 __global__ void k_scatter_adjacency(int64_t nv, const int64_t* __restrict__ off, const int64_t* __restrict__ adj,
-                                    const int64_t* __restrict__ row, int32_t* __restrict__ col)
+                                    const int64_t* __restrict__ row, int32_t* __restrict__ col,
+                                    unsigned long long* skew)
 {
     const int lane = threadIdx.x & 31;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    unsigned long long sum = 0;
     for (int64_t v = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < nv; v += nw) {
         const int64_t b = off[v], d = off[v + 1] - b, r = row[v];
-        for (int64_t i = lane; i < d; i += 32) col[r + i] = (int32_t)adj[b + i];
+        for (int64_t i = lane; i < d; i += 32) {
+            const int32_t c = (int32_t)adj[b + i];
+            col[r + i] = c;
+            sum += edge_mix((int)v, c);
+        }
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0 && sum) atomicAdd(skew, sum);
 }
 
 // Warp per listed vertex of at most 32 neighbours: bitonic sort in registers.
@@ -130,9 +140,10 @@ __global__ void __launch_bounds__(kSortNT) k_sort_long(const int32_t* __restrict
 // vertex's neighbours, each list sorted.  Synchronous on stream s.
 cudaError_t build_adjacency(int64_t nv, const int64_t* off, const int64_t* adj, const int64_t* d_row,
                             const int32_t* d_deg, const std::vector<int32_t>& deg, int32_t* d_col, int sm_count,
-                            cudaStream_t s)
+                            cudaStream_t s, unsigned long long* skew)
 {
     const int64_t ne = off[nv];
+    unsigned long long* d_skew = nullptr;
     cudaError_t e;
     int64_t *d_off = nullptr, *d_adj = nullptr, *d_tmp_off = nullptr;
     int32_t *d_short = nullptr, *d_long = nullptr, *d_tmp = nullptr;
@@ -153,7 +164,8 @@ cudaError_t build_adjacency(int64_t nv, const int64_t* off, const int64_t* adj, 
         }
     }
     auto cleanup = [&]() {
-        for (void* p : {(void*)d_off, (void*)d_adj, (void*)d_tmp_off, (void*)d_short, (void*)d_long, (void*)d_tmp})
+        for (void* p : {(void*)d_off, (void*)d_adj, (void*)d_tmp_off, (void*)d_short, (void*)d_long, (void*)d_tmp,
+                        (void*)d_skew})
             if (p) cudaFree(p);
     };
     if ((e = cudaMalloc(&d_off, sizeof(int64_t) * (nv + 1))) ||
@@ -162,6 +174,7 @@ cudaError_t build_adjacency(int64_t nv, const int64_t* off, const int64_t* adj, 
         (e = cudaMalloc(&d_long, sizeof(int32_t) * std::max<size_t>(longl.size(), 1))) ||
         (e = cudaMalloc(&d_tmp_off, sizeof(int64_t) * std::max<size_t>(tmp_off.size(), 1))) ||
         (e = cudaMalloc(&d_tmp, sizeof(int32_t) * std::max<int64_t>(tmp_total, 1))) ||
+        (e = cudaMalloc(&d_skew, sizeof *d_skew)) || (e = cudaMemsetAsync(d_skew, 0, sizeof *d_skew, s)) ||
         (e = cudaMemcpyAsync(d_off, off, sizeof(int64_t) * (nv + 1), cudaMemcpyHostToDevice, s)) ||
         (ne && (e = cudaMemcpyAsync(d_adj, adj, sizeof(int64_t) * ne, cudaMemcpyHostToDevice, s))) ||
         (!shortl.empty() &&
@@ -174,12 +187,14 @@ cudaError_t build_adjacency(int64_t nv, const int64_t* off, const int64_t* adj, 
         return e;
     }
     const int grid = sm_count * 8;
-    if (nv) k_scatter_adjacency<<<grid, 256, 0, s>>>(nv, d_off, d_adj, d_row, d_col);
+    if (nv) k_scatter_adjacency<<<grid, 256, 0, s>>>(nv, d_off, d_adj, d_row, d_col, d_skew);
     if (!shortl.empty()) k_sort_short<<<grid, 256, 0, s>>>(d_short, (int)shortl.size(), d_row, d_deg, d_col);
     if (!longl.empty())
         k_sort_long<<<(int)std::min<size_t>(longl.size(), (size_t)sm_count * 4), kSortNT, 0, s>>>(
             d_long, (int)longl.size(), d_row, d_deg, d_col, d_tmp, d_tmp_off);
-    if ((e = cudaGetLastError()) || (e = cudaStreamSynchronize(s))) {
+    if ((e = cudaGetLastError()) ||
+        (e = cudaMemcpyAsync(skew, d_skew, sizeof *skew, cudaMemcpyDeviceToHost, s)) ||
+        (e = cudaStreamSynchronize(s))) {
         cleanup();
         return e;
     }

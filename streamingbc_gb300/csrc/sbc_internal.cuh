@@ -198,6 +198,19 @@ __device__ __forceinline__ bool has_edge(const DevGraph& G, int x, int64_t rx, i
     return false;
 }
 
+// A mix of the directed edge u -> v with edge_mix(u, v) == -edge_mix(v, u): its
+// sum over an adjacency (the edge skew) is 0 when every edge is stored in both
+// directions, and with overwhelming probability only then.
+__host__ __device__ __forceinline__ unsigned long long edge_mix(int u, int v)
+{
+    const int a = u < v ? u : v, b = u < v ? v : u;
+    unsigned long long h = ((unsigned long long)(unsigned)a << 32 | (unsigned)b) * 0x9e3779b97f4a7c15ull;
+    h ^= h >> 29;
+    h *= 0xbf58476d1ce4e5b9ull;
+    h ^= h >> 32;
+    return u == v ? 0ull : u < v ? h : 0ull - h;
+}
+
 __device__ __forceinline__ uint8_t enc_d8(int d)
 {
     return d == SBC_INF ? (uint8_t)SBC_D8_INF : (d >= SBC_D8_DEEP ? (uint8_t)SBC_D8_DEEP : (uint8_t)d);

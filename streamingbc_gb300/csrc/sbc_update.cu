@@ -378,21 +378,24 @@ cudaError_t launch_delete_finish(sbc_forest* f)
     if (n == 0) return cudaSuccess;
     // a few roots of a large graph: one at a time by the whole GPU (a CTA
     // would walk the whole graph alone); otherwise a CTA per root
-    if (n <= kWideRecompute && f->nv >= kWideRecomputeMinVertices) {
+    const bool wide = n <= kWideRecompute && f->nv >= kWideRecomputeMinVertices;
+    if (wide) {
         std::vector<int> rows(n);
         if ((e = cudaMemcpyAsync(rows.data(), f->d_dlist, sizeof(int) * n, cudaMemcpyDeviceToHost, s)) ||
             (e = cudaStreamSynchronize(s)))
             return e;
         if ((e = recompute_roots_wide(f, rows, f->d_dlist))) return e;
-    } else if ((e = launch_static_list(f, f->d_dlist, f->d_dcnt))) {
+    } else if ((e = launch_static_list(f, f->d_dlist, f->d_dcnt, n))) {
         return e;
     }
     const dim3 grid((unsigned)std::min<int64_t>((f->nv + 255) / 256, 64), (unsigned)std::min<int64_t>(f->nk, 4096));
     k_bc_rows<<<grid, 256, 0, s>>>(f->d_delta, f->d_roots, f->d_dlist, f->d_dcnt, f->nv, f->d_bc, 1.0);
     if ((e = cudaGetLastError())) return e;
-    if ((e = launch_dist2_rows(f, f->d_dlist, f->d_dcnt))) return e;
-    if ((e = launch_level_hist_list(f, f->d_dlist, f->d_dcnt))) return e;
-    if ((e = launch_roster_build_list(f, f->d_dlist, f->d_dcnt))) return e;
+    // what the static kernel derives from the levels itself
+    if (wide && ((e = launch_dist2_rows(f, f->d_dlist, f->d_dcnt)) ||
+                 (e = launch_level_hist_list(f, f->d_dlist, f->d_dcnt)) ||
+                 (e = launch_roster_build_list(f, f->d_dlist, f->d_dcnt))))
+        return e;
     k_clear_dirty<<<(int)std::min<int64_t>((f->nk + 255) / 256, 64), 256, 0, s>>>(f->d_dlist, f->d_dcnt, f->d_dirty);
     if ((e = cudaGetLastError())) return e;
     return cudaMemsetAsync(f->d_dcnt, 0, sizeof(int), s);
