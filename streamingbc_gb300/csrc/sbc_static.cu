@@ -15,6 +15,7 @@
 #include <climits>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include "sbc_gb300.h"
 #include "sbc_host.h"
 #include "sbc_internal.cuh"
@@ -38,6 +39,7 @@ struct StaticArgs {
     int32_t* roster_dirty;
     ScratchBase scr;
     int halves;        // static workers per update worker's scratch (1 or 2)
+    int third_bits;    // kBits: a third bitmap in shared memory, not in scr.st
     int* work_counter;
     unsigned long long* counters;  // [0] vertices, [1] edges
     const int* list;   // roots to (re)compute, or null for all
@@ -48,184 +50,280 @@ struct StaticArgs {
 };
 
 // Where one root's working set lives.
-//   kSmall   the whole row (levels, sigma, child weights, queue) and both
+//   kSmall   the whole row (levels, sigma, child weights, queue) and the three
 //            bitmaps in shared memory; results are written out once
-//   kBits    rows in HBM, both bitmaps in shared memory
-//   kOneBits the tested bitmap in shared memory, the visited one in HBM
-//   kNoBits  both bitmaps in HBM
+//   kBits    rows in HBM, bitmaps in shared memory (the one that only a pull
+//            writes in HBM: what shared memory leaves is the L1 cache, which
+//            the walks of short lists live on)
+//   kOneBits the tested bitmap in shared memory, the other two in HBM
+//   kNoBits  all bitmaps in HBM
 enum StaticMode { kSmall = 0, kBits = 1, kOneBits = 2, kNoBits = 3 };
 
 constexpr int kSlotLevels = 64;   // levels whose slot counts the backward pass can compare
-constexpr int kThreadDeg = 4;     // up to this degree a vertex is one thread's work,
-constexpr int kGroupDeg = 64;     // up to this eight lanes',
-constexpr int kBigDeg = 16384;    // up to this a warp's, and the CTA's beyond
-constexpr int kBigCap = 64;       // CTA-wide vertices listed per walk (the others stay a warp's)
+// A vertex is scanned by one lane up to 8 neighbours, by 4 lanes up to 32, by
+// 16 up to 128 (each lane then has 8 at a time in flight), by the warp up to
+// kBigDeg, and beyond in segments of kSegSlots that the CTA's warps share out.
+constexpr int kLaneSlots = 8;
+constexpr int kBigDeg = 1024;
+constexpr int kSegSlots = 2048;
+// Such vertices listed per walk (the others stay a warp's).
+constexpr int kBigCap = 1024, kBigCapSmall = 64;
 
-template <int NT>
+template <int NT, int CAP>
 struct StaticSmem {
-    int item, tail, next, nbig;
+    static constexpr int kCap = CAP;
+    int item, tail, next, next_seg, nbig;
     unsigned long long slots, total;
     unsigned long long lvslots[kSlotLevels];
-    int big[kBigCap];
-    int bighit[kBigCap];
+    int big[CAP];
+    int seg_end[CAP];  // running segment counts of big[]
+    unsigned char bighit[CAP];
     int buf[NT / 32][64];
+    unsigned char order[NT / 32][32];
+    int wsum[NT / 32];
     unsigned long long walked_v, walked_e, scanned;
 };
 
 __device__ __forceinline__ bool bit_of(const uint32_t* B, int k) { return (B[k >> 5] >> (k & 31)) & 1u; }
 
-__device__ __forceinline__ int nth_group(unsigned m, int g)
+// Neighbours s0, s0 + step, ... of a list of d slots at rs (-1 past its end).
+__device__ __forceinline__ void load_slots(const DevGraph& G, int64_t rs, int d, int s0, int step, int (&k)[kLaneSlots])
 {
-    for (int q = 0; q < g; ++q) m &= m - 1;  // drops the g lowest set bits
-    return m ? __ffs(m) - 1 : -1;
+#pragma unroll
+    for (int u = 0; u < kLaneSlots; ++u) k[u] = s0 + step * u < d ? G.col[rs + s0 + step * u] : -1;
 }
 
-// One vertex per lane (x where ok): act(v, k[4]) gets up to four neighbours k
-// (-1 past the end) of a vertex whose value is v, from whichever lane scans
-// them: short lists stay with their lane, up to kGroupDeg eight lanes share
-// one, longer ones take the warp, and lists of kBigDeg and more are listed in
-// sm.big for the whole CTA.  No block barrier inside.
-template <int NT, class V, class Act>
-__device__ __forceinline__ void push_batch(const DevGraph& G, StaticSmem<NT>& sm, int x, bool ok, V v, Act act)
+// Bit u: k[u] is a neighbour (>= 0) and in bitmap B.  All words are loaded
+// before any is tested.
+__device__ __forceinline__ unsigned in_bitmap(const uint32_t* B, const int (&k)[kLaneSlots])
+{
+    unsigned w[kLaneSlots];
+#pragma unroll
+    for (int u = 0; u < kLaneSlots; ++u) w[u] = B[max(k[u], 0) >> 5];
+    unsigned in = 0;
+#pragma unroll
+    for (int u = 0; u < kLaneSlots; ++u) in |= (k[u] >= 0 ? (w[u] >> (k[u] & 31)) & 1u : 0u) << u;
+    return in;
+}
+
+// Bit u: k[u] is a neighbour.
+__device__ __forceinline__ unsigned present(const int (&k)[kLaneSlots])
+{
+    unsigned in = 0;
+#pragma unroll
+    for (int u = 0; u < kLaneSlots; ++u) in |= (k[u] >= 0 ? 1u : 0u) << u;
+    return in;
+}
+
+// s += val[k[u]] over the k[u] in bitmap B; returns their bits.  Every
+// neighbour is tested, then the values are gathered, then summed.
+template <class T>
+__device__ __forceinline__ unsigned sum_in(const uint32_t* B, const T* val, const int (&k)[kLaneSlots], T& s)
+{
+    const unsigned in = in_bitmap(B, k);
+    T y[kLaneSlots];
+#pragma unroll
+    for (int u = 0; u < kLaneSlots; ++u) y[u] = (in >> u) & 1u ? val[k[u]] : (T)0;
+#pragma unroll
+    for (int u = 0; u < kLaneSlots; ++u)
+        if ((in >> u) & 1u) s += y[u];
+    return in;
+}
+
+// Appends k[u] for every set bit u of each calling lane's `first`: the lanes
+// here reserve the queue's slots together.
+template <class Sm>
+__device__ __forceinline__ void append_first(Sm& sm, int32_t* q, const int (&k)[kLaneSlots], unsigned first)
+{
+    const unsigned act = __activemask();
+    if (!__any_sync(act, first)) return;
+    const unsigned below = (1u << (threadIdx.x & 31)) - 1u;
+    int total = 0, at[kLaneSlots];
+#pragma unroll
+    for (int u = 0; u < kLaneSlots; ++u) {
+        const unsigned m = __ballot_sync(act, (first >> u) & 1u);
+        at[u] = total + __popc(m & below);
+        total += __popc(m);
+    }
+    const int leader = __ffs(act) - 1;
+    int base = 0;
+    if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(&sm.tail, total);
+    base = __shfl_sync(act, base, leader);
+#pragma unroll
+    for (int u = 0; u < kLaneSlots; ++u)
+        if ((first >> u) & 1u) q[base + at[u]] = k[u];
+}
+
+// *p += v in shared memory, modulo 2^64, as a 32-bit add and a carry: a 64-bit
+// shared add is a compare-and-swap loop.
+__device__ __forceinline__ void add_shared(int64_t* p, long long v)
+{
+    const unsigned lo = (unsigned)v;
+    const unsigned old = atomicAdd((unsigned*)p, lo);
+    const unsigned hi = (unsigned)((unsigned long long)v >> 32) + (old + lo < old ? 1u : 0u);
+    if (hi) atomicAdd((unsigned*)p + 1, hi);
+}
+
+// a / s.  The SM issues one fp64 instruction per 16 cycles, and a division by
+// the compiler takes more of them than all else done per vertex: here the
+// reciprocal starts from the fp32 one (24 bits), one Newton step doubles its
+// bits, and the quotient's remainder, exact by fused multiply-add, corrects the
+// quotient to the last bit (Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", 1990): five fp64 instructions.
+__device__ __forceinline__ double child_weight(double a, int64_t s)
+{
+    const double b = (double)s;
+    // s <= 0 (a sum that wrapped) and values that are not finite: plain division
+    if (s <= 0 || (unsigned)__double2hiint(a) >= 0x7fd00000u) return a / b;
+    const int f = __float_as_int(__frcp_rn(__ll2float_rn(s)));
+    const double r = __hiloint2double((f >> 3) + (896 << 20), f << 29);  // the float's value
+    const double r1 = fma(r, fma(-b, r, 1.0), r);
+    const double q = a * r1;
+    return fma(fma(-b, q, a), r1, q);
+}
+
+// A vertex held by one lane of a task: its slots and its value.
+template <class V>
+struct TaskVertex {
+    int x, d;
+    int64_t rs;
+    V v;
+};
+
+// The task's vertices of degree (lo, hi], W lanes each: f(owner lane j or -1,
+// rs, d, v, step's first rank) for 32 / W of them at a time, all lanes calling.
+template <int W, class Sm, class V, class F>
+__device__ __forceinline__ void lane_groups(Sm& sm, const TaskVertex<V>& q, int lo, int hi, F f)
 {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    int64_t rs = 0;
-    int d = 0;
-    if (ok) {
-        rs = G.row[x];
-        d = G.deg[x];
-    }
-    if (d >= kBigDeg) {
-        const int p = atomicAdd(&sm.nbig, 1);
-        if (p < kBigCap) {
-            sm.big[p] = x;
-            d = 0;
-        }
-    }
-    if (d > 0 && d <= kThreadDeg) {
-        int k[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) k[u] = u < d ? G.col[rs + u] : -1;
-        act(v, k);
+    unsigned char* order = sm.order[threadIdx.x >> 5];
+    const bool mine = q.d > lo && q.d <= hi;
+    const unsigned m = __ballot_sync(full, mine);
+    if (!m) return;
+    const int n = __popc(m), rank = __popc(m & ((1u << lane) - 1u));
+    if (mine) order[rank] = (unsigned char)lane;
+    __syncwarp();
+    for (int t = 0; t < n; t += 32 / W) {
+        const int at = t + lane / W;
+        const int j = at < n ? order[at] : -1;
+        const int64_t rj = __shfl_sync(full, q.rs, j & 31);
+        const int dj = __shfl_sync(full, q.d, j & 31);
+        const V vj = __shfl_sync(full, q.v, j & 31);
+        f(j, rj, dj, vj, mine ? rank - t : -1);
     }
     __syncwarp();
-    for (unsigned m = __ballot_sync(full, d > kThreadDeg && d <= kGroupDeg); m;) {
-        const int j = nth_group(m, lane >> 3);
-        const int64_t rj = __shfl_sync(full, rs, j & 31);
-        const int dj = __shfl_sync(full, d, j & 31);
-        const V vj = __shfl_sync(full, v, j & 31);
-        if (j >= 0)
-            for (int s0 = lane & 7; s0 < dj; s0 += 32) {
-                int k[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) k[u] = s0 + 8 * u < dj ? G.col[rj + s0 + 8 * u] : -1;
-                act(vj, k);
-            }
-        __syncwarp();
-        for (int q = 0; q < 4; ++q) m &= m - 1;
+}
+
+// One vertex per lane (none where q.d is 0): act(v, k[]) gets the neighbours k
+// (-1: none) of a vertex whose value is v, from whichever lane scans them.
+// Vertices of degree kBigDeg and more are listed for big_segments.  No block
+// barrier inside.
+template <class Sm, class V, class Act>
+__device__ __forceinline__ void push_batch(const DevGraph& G, Sm& sm, TaskVertex<V> q, Act act)
+{
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    if (q.d >= kBigDeg) {
+        const int p = atomicAdd(&sm.nbig, 1);
+        if (p < Sm::kCap) {
+            sm.big[p] = q.x;
+            q.d = 0;
+        }
     }
-    for (unsigned m = __ballot_sync(full, d > kGroupDeg); m; m &= m - 1) {
+    int k[kLaneSlots];
+    if (q.d > 0 && q.d <= kLaneSlots) {
+        load_slots(G, q.rs, q.d, 0, 1, k);
+        act(q.v, k);
+    }
+    __syncwarp();
+    lane_groups<4>(sm, q, kLaneSlots, 4 * kLaneSlots, [&](int j, int64_t rj, int dj, V vj, int) {
+        if (j >= 0) {
+            load_slots(G, rj, dj, lane & 3, 4, k);
+            act(vj, k);
+        }
+        __syncwarp();
+    });
+    lane_groups<16>(sm, q, 4 * kLaneSlots, 16 * kLaneSlots, [&](int j, int64_t rj, int dj, V vj, int) {
+        if (j >= 0) {
+            load_slots(G, rj, dj, lane & 15, 16, k);
+            act(vj, k);
+        }
+        __syncwarp();
+    });
+    for (unsigned m = __ballot_sync(full, q.d > 16 * kLaneSlots); m; m &= m - 1) {
         const int j = __ffs(m) - 1;
-        const int64_t rj = __shfl_sync(full, rs, j);
-        const int dj = __shfl_sync(full, d, j);
-        const V vj = __shfl_sync(full, v, j);
-        for (int s0 = lane; s0 < dj; s0 += 128) {
-            int k[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) k[u] = s0 + 32 * u < dj ? G.col[rj + s0 + 32 * u] : -1;
+        const int64_t rj = __shfl_sync(full, q.rs, j);
+        const int dj = __shfl_sync(full, q.d, j);
+        const V vj = __shfl_sync(full, q.v, j);
+        for (int s0 = lane; s0 < dj; s0 += 32 * kLaneSlots) {
+            load_slots(G, rj, dj, s0, 32, k);
             act(vj, k);
         }
         __syncwarp();
     }
 }
 
-// One vertex per lane: sums val(k) over the neighbours k with test(k), the
+// One vertex per lane: sums val[k] over the neighbours k in bitmap B, the
 // lists shared out as in push_batch, and calls done(x, sum, whether any
 // neighbour passed) in the lane that brought x.
-template <int NT, class T, class Test, class Val, class Done>
-__device__ __forceinline__ void pull_batch(const DevGraph& G, StaticSmem<NT>& sm, int x, bool ok, Test test, Val val,
-                                           Done done)
+template <class T, class Sm, class Done>
+__device__ __forceinline__ void pull_batch(const DevGraph& G, Sm& sm, TaskVertex<int> q, bool ok,
+                                           const uint32_t* B, const T* val, Done done)
 {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    int64_t rs = 0;
-    int d = 0;
-    if (ok) {
-        rs = G.row[x];
-        d = G.deg[x];
-    }
-    if (d >= kBigDeg) {
+    if (q.d >= kBigDeg) {
         const int p = atomicAdd(&sm.nbig, 1);
-        if (p < kBigCap) {
-            sm.big[p] = x;
+        if (p < Sm::kCap) {
+            sm.big[p] = q.x;
             sm.bighit[p] = 0;
-            d = 0;
-            ok = false;  // finished by the whole CTA
+            q.d = 0;
+            ok = false;  // finished after big_segments
         }
     }
-    // four neighbours tested, then their values gathered, then summed
-    auto four = [&](const int (&k)[4], T& s, bool& hit) {
-        bool t[4];
-        T y[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) t[u] = k[u] >= 0 && test(k[u]);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) y[u] = t[u] ? val(k[u]) : (T)0;
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (t[u]) {
-                s += y[u];
-                hit = true;
-            }
-    };
+    int k[kLaneSlots];
+    auto add = [&](T& s, bool& hit) { hit |= sum_in(B, val, k, s) != 0u; };
     T sum = (T)0;
     bool hit = false;
-    if (d > 0 && d <= kThreadDeg) {
-        int k[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) k[u] = u < d ? G.col[rs + u] : -1;
-        four(k, sum, hit);
+    if (q.d > 0 && q.d <= kLaneSlots) {
+        load_slots(G, q.rs, q.d, 0, 1, k);
+        add(sum, hit);
     }
     __syncwarp();
-    for (unsigned m = __ballot_sync(full, d > kThreadDeg && d <= kGroupDeg); m;) {
-        const int j = nth_group(m, lane >> 3);
-        const int64_t rj = __shfl_sync(full, rs, j & 31);
-        const int dj = __shfl_sync(full, d, j & 31);
-        T s = (T)0;
-        bool h = false;
-        if (j >= 0)
-            for (int s0 = lane & 7; s0 < dj; s0 += 32) {
-                int k[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) k[u] = s0 + 8 * u < dj ? G.col[rj + s0 + 8 * u] : -1;
-                four(k, s, h);
+    auto grouped = [&](auto width, int lo, int hi) {
+        constexpr int W = decltype(width)::value;
+        lane_groups<W>(sm, q, lo, hi, [&](int j, int64_t rj, int dj, int, int ahead) {
+            T s = (T)0;
+            bool h = false;
+            if (j >= 0) {
+                load_slots(G, rj, dj, lane & (W - 1), W, k);
+                add(s, h);
             }
-        const unsigned hits = __ballot_sync(full, h);
-        if (hits) {
+            const unsigned hits = __ballot_sync(full, h);
+            if (hits) {
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(full, s, o);
-        }
-        // the vertex's own lane takes its group's total
-        const int rank = __popc(m & ((1u << lane) - 1u));
-        const T mine = __shfl_sync(full, s, (rank & 3) * 8);
-        if (((m >> lane) & 1u) && rank < 4) {
-            sum = mine;
-            hit = (hits >> (rank * 8)) & 0xffu;
-        }
-        for (int q = 0; q < 4; ++q) m &= m - 1;
-    }
-    for (unsigned m = __ballot_sync(full, d > kGroupDeg); m; m &= m - 1) {
+                for (int o = W / 2; o > 0; o >>= 1) s += __shfl_xor_sync(full, s, o);
+                // the vertex's own lane takes its group's total
+                const T mine = __shfl_sync(full, s, (ahead * W) & 31);
+                if (ahead >= 0 && ahead < 32 / W) {
+                    sum = mine;
+                    hit = (hits >> (ahead * W)) & ((1u << W) - 1u);
+                }
+            }
+        });
+    };
+    grouped(std::integral_constant<int, 4>(), kLaneSlots, 4 * kLaneSlots);
+    grouped(std::integral_constant<int, 16>(), 4 * kLaneSlots, 16 * kLaneSlots);
+    for (unsigned m = __ballot_sync(full, q.d > 16 * kLaneSlots); m; m &= m - 1) {
         const int j = __ffs(m) - 1;
-        const int64_t rj = __shfl_sync(full, rs, j);
-        const int dj = __shfl_sync(full, d, j);
+        const int64_t rj = __shfl_sync(full, q.rs, j);
+        const int dj = __shfl_sync(full, q.d, j);
         T s = (T)0;
         bool h = false;
-        for (int s0 = lane; s0 < dj; s0 += 128) {
-            int k[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) k[u] = s0 + 32 * u < dj ? G.col[rj + s0 + 32 * u] : -1;
-            four(k, s, h);
+        for (int s0 = lane; s0 < dj; s0 += 32 * kLaneSlots) {
+            load_slots(G, rj, dj, s0, 32, k);
+            add(s, h);
         }
         if (__any_sync(full, h)) {
 #pragma unroll
@@ -236,59 +334,146 @@ __device__ __forceinline__ void pull_batch(const DevGraph& G, StaticSmem<NT>& sm
             }
         }
     }
-    if (ok) done(x, sum, hit);
+    if (ok) done(q.x, sum, hit);
     __syncwarp();
 }
 
 // Vertices of a list, handed to the warps in tasks of up to 32 (fewer when the
-// list is short, so that every warp has work); batch(x, ok) per warp.
-template <int NT, class Batch>
-__device__ __forceinline__ void list_tasks(StaticSmem<NT>& sm, const int32_t* list, int n, Batch batch)
+// list is short, so that every warp has work); batch(task vertex, ok) per
+// warp.  The next task's slots and value(x) are loaded before the current one
+// is walked.
+template <int NT, class V, class Sm, class Value, class Batch>
+__device__ __forceinline__ void list_tasks(const DevGraph& G, Sm& sm, const int32_t* list, int n,
+                                           unsigned long long slots, Value value, Batch batch)
 {
     const int lane = threadIdx.x & 31;
-    const int t = min(32, max(1, (n + NT / 32 - 1) / (NT / 32)));
-    for (;;) {
+    int t = min(32, max(1, (n + NT / 32 - 1) / (NT / 32)));
+    // about kSegSlots * 2 slots a task: lists come in vertex order, which
+    // gathers the hubs of some graphs in a few tasks
+    if (slots > 64ull * n) t = min(t, max(4, (int)(2ull * kSegSlots * n / slots)));
+    auto claim = [&](TaskVertex<V>& q, bool& ok) {
         int base = 0;
         if (lane == 0) base = atomicAdd(&sm.next, t);
         base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= n) break;
-        const bool ok = lane < t && base + lane < n;
-        batch(ok ? list[base + lane] : 0, ok);
+        ok = lane < t && base + lane < n;
+        q.x = q.d = 0;
+        q.rs = 0;
+        q.v = (V)0;
+        if (ok) {
+            q.x = list[base + lane];
+            q.rs = G.row[q.x];
+            q.d = G.deg[q.x];
+            q.v = value(q.x);
+        }
+        return base < n;
+    };
+    TaskVertex<V> q;
+    bool ok;
+    for (bool more = claim(q, ok); more;) {
+        TaskVertex<V> q2;
+        bool ok2;
+        more = claim(q2, ok2);
+        batch(q, ok);
+        q = q2;
+        ok = ok2;
     }
 }
 
+// The walk's listed long vertices, a segment per warp at a time, once every
+// task is done: seg(i, x, rs, s0, s1) walks slots [s0, s1) of vertex x =
+// big[i].  Called by the whole CTA, with block barriers; returns how many
+// vertices are listed.
+template <class Sm, class Seg>
+__device__ __forceinline__ int big_segments(const DevGraph& G, Sm& sm, Seg seg)
+{
+    __syncthreads();
+    const int nb = min(sm.nbig, Sm::kCap);
+    if (nb == 0) return 0;
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x < 32) {
+        int run = 0;
+        for (int i0 = 0; i0 < nb; i0 += 32) {
+            int c = i0 + lane < nb ? (G.deg[sm.big[i0 + lane]] + kSegSlots - 1) / kSegSlots : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(full, c, o);
+                if (lane >= o) c += y;
+            }
+            if (i0 + lane < nb) sm.seg_end[i0 + lane] = run + c;
+            run += __shfl_sync(full, c, 31);
+        }
+        if (lane == 0) sm.next_seg = 0;
+    }
+    __syncthreads();
+    for (;;) {
+        int u = 0;
+        if (lane == 0) u = atomicAdd(&sm.next_seg, 1);
+        u = __shfl_sync(full, u, 0);
+        if (u >= sm.seg_end[nb - 1]) break;
+        int lo = 0, hi = nb - 1;  // first i with seg_end[i] > u
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (sm.seg_end[mid] > u) hi = mid;
+            else lo = mid + 1;
+        }
+        const int x = sm.big[lo];
+        const int d = G.deg[x];
+        const int s0 = (u - (lo ? sm.seg_end[lo - 1] : 0)) * kSegSlots;
+        seg(lo, x, G.row[x], s0, min(d, s0 + kSegSlots));
+    }
+    return nb;
+}
+
 // The vertices whose bit in V is clear, packed 32 at a time per warp.
-template <int NT, class Batch>
-__device__ __forceinline__ void unset_tasks(StaticSmem<NT>& sm, const uint32_t* V, int nw, Batch batch)
+template <int NT, class Sm, class Batch>
+__device__ __forceinline__ void unset_tasks(const DevGraph& G, Sm& sm, const uint32_t* V, int nw,
+                                            Batch batch)
 {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     int* buf = sm.buf[threadIdx.x >> 5];
     const int t = min(32, max(1, nw / (NT / 32)));
-    int pend = 0;
+    int pend = 0, base = 0;
+    unsigned mine = 0, have = 0;  // the claimed words, and which lanes' words still have vertices to take
+    bool more = true, held = false, ok = false;
+    TaskVertex<int> q{0, 0, 0, 0};
     for (;;) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(&sm.next, t);
-        base = __shfl_sync(full, base, 0);
-        if (base >= nw) break;
-        const unsigned mine = lane < t && base + lane < nw ? ~V[base + lane] : 0u;
-        for (unsigned have = __ballot_sync(full, mine != 0u); have; have &= have - 1) {
+        while (pend < 32 && (more || have)) {
+            if (!have) {
+                if (lane == 0) base = atomicAdd(&sm.next, t);
+                base = __shfl_sync(full, base, 0);
+                more = base < nw;
+                mine = more && lane < t && base + lane < nw ? ~V[base + lane] : 0u;
+                have = __ballot_sync(full, mine != 0u);
+                continue;
+            }
             const int j = __ffs(have) - 1;
+            have &= have - 1;
             const unsigned w = __shfl_sync(full, mine, j);
             if ((w >> lane) & 1u) buf[pend + __popc(w & ((1u << lane) - 1u))] = (base + j) * 32 + lane;
             pend += __popc(w);
             __syncwarp();
-            if (pend >= 32) {
-                batch(buf[lane], true);
-                pend -= 32;
-                const int rest = buf[32 + lane];
-                __syncwarp();
-                if (lane < pend) buf[lane] = rest;
-                __syncwarp();
-            }
         }
+        // the batch's slots are loaded now and walked after the one before it
+        const bool ok2 = lane < pend;
+        TaskVertex<int> q2{ok2 ? buf[lane] : 0, 0, 0, 0};
+        if (ok2) {
+            q2.rs = G.row[q2.x];
+            q2.d = G.deg[q2.x];
+        }
+        const int left = max(pend - 32, 0);
+        const int rest = lane < left ? buf[32 + lane] : 0;
+        __syncwarp();
+        if (lane < left) buf[lane] = rest;
+        __syncwarp();
+        if (held) batch(q, ok);
+        if (pend == 0) break;
+        pend = left;
+        q = q2;
+        ok = ok2;
+        held = true;
     }
-    if (pend > 0) batch(lane < pend ? buf[lane] : 0, lane < pend);
 }
 
 // Static Brandes of one root per CTA at a time.
@@ -312,7 +497,8 @@ template <int NT, int MODE>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant__ StaticArgs A)
 {
     extern __shared__ __align__(16) unsigned char s_dyn[];
-    __shared__ StaticSmem<NT> sm;
+    using Sm = StaticSmem<NT, MODE == kSmall ? kBigCapSmall : kBigCap>;
+    __shared__ Sm sm;
     if (A.abort && *A.abort) return;
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -324,7 +510,10 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
     const size_t slot = blockIdx.x / A.halves;
     int32_t *qd, *lvl;
     double* acc;
-    uint32_t *B, *V;  // tested bitmap, visited bitmap (isolated vertices count as visited)
+    // the tested bitmap; the visited vertices (isolated ones count as visited);
+    // the vertices claimed for the next level, by a push and by a pull (which
+    // sets each word from one warp alone and needs no fast bitmap for it)
+    uint32_t *B, *V, *Npush, *Npull;
     int32_t* sD = nullptr;
     int64_t* sS = nullptr;
     if (MODE == kSmall) {
@@ -341,6 +530,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
         p += 4 * nv;
         V = (uint32_t*)p;
         B = V + nw;
+        Npush = Npull = B + nw;
     } else {
         const bool second = blockIdx.x % A.halves;
         qd = (second ? A.scr.qa : A.scr.qd) + slot * nv;
@@ -348,13 +538,20 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
         acc = (second ? (double*)A.scr.dp : A.scr.acc) + slot * nv;
         if (MODE == kBits) {
             V = (uint32_t*)s_dyn;
-            B = V + nw;
+            B = Npush = V + nw;
+            Npull = A.third_bits ? B + nw : (uint32_t*)(A.scr.st + slot * nv) + (second ? nw : 0);
         } else {
             V = A.scr.bits + slot * bitmap_words(nv);
-            B = MODE == kOneBits ? (uint32_t*)s_dyn : (uint32_t*)(A.scr.st + slot * nv);
+            Npush = Npull = (uint32_t*)(A.scr.st + slot * nv);
+            B = MODE == kOneBits ? (uint32_t*)s_dyn : (uint32_t*)(A.scr.qa + slot * nv);
         }
     }
     if (threadIdx.x == 0) sm.walked_v = sm.walked_e = sm.scanned = 0;
+    // the others are kept zero between launches where they are in HBM
+    for (int i = threadIdx.x; i < nw; i += NT) {
+        B[i] = 0u;
+        if (MODE == kSmall || A.third_bits) Npull[i] = 0u;
+    }
 
     for (;;) {
         if (threadIdx.x == 0) {
@@ -418,110 +615,155 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                 const unsigned long long rest = total - visited;
                 // the scan for unvisited vertices itself costs about a slot per four vertices
                 const bool pull = sym && rest + (unsigned long long)(nv >> 2) < front;
+                // a level that may have more vertices than the bitmap has words
+                // is listed from N when it is complete, in vertex order
+                const bool dense = pull || front >= (unsigned)nw;
+                uint32_t* const N = pull ? Npull : Npush;
                 if (threadIdx.x == 0) sm.next = sm.nbig = 0;
                 __syncthreads();
                 if (threadIdx.x == 0) sm.slots = 0;
                 if (!pull) {
                     scanned += front;
-                    const uint32_t* T = V;
-                    if (MODE == kOneBits) {
-                        if (!held) {
-                            for (int i = threadIdx.x; i < nw; i += NT) B[i] = V[i];
-                            held = true;
-                            __syncthreads();
-                        }
-                        T = B;
+                    const uint32_t* T = MODE == kOneBits ? B : V;
+                    if (MODE == kOneBits && !held) {
+                        for (int i = threadIdx.x; i < nw; i += NT) B[i] = V[i];
+                        held = true;
+                        __syncthreads();
                     }
-                    // an unvisited neighbour gains x's sigma; the first visitor
-                    // (the one that finds sigma 0) claims it for the level.  A
-                    // sum that wraps to 0 only makes more of them try.
-                    auto act = [&](long long s, const int (&k)[4]) {
-                        bool t[4];
-                        unsigned long long old[4];
+                    // An unvisited neighbour gains x's sigma and joins N; where
+                    // the level is short its first visitor, the one that sets
+                    // the bit, also lists it.
+                    auto act = [&](long long s, const int (&k)[kLaneSlots]) {
+                        const unsigned in = present(k) & ~in_bitmap(T, k);
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) t[u] = k[u] >= 0 && !bit_of(T, k[u]);
+                        for (int u = 0; u < kLaneSlots; ++u)
+                            if ((in >> u) & 1u) {
+                                if (MODE == kSmall) add_shared(&Sg[k[u]], s);
+                                else atomic_add_i64(&Sg[k[u]], s);
+                            }
+                        unsigned first = in & ~in_bitmap(N, k);
+                        if (dense) {
 #pragma unroll
-                        for (int u = 0; u < 4; ++u)
-                            old[u] = t[u] ? atomicAdd((unsigned long long*)&Sg[k[u]], (unsigned long long)s) : 1ull;
-#pragma unroll
-                        for (int u = 0; u < 4; ++u)
-                            if (old[u] == 0ull)
-                                warp_append(&sm.tail, qd, k[u], atomicCAS(&D[k[u]], SBC_INF, L + 1) == SBC_INF);
-                    };
-                    list_tasks<NT>(sm, qd + lo, hi - lo, [&](int x, bool ok) {
-                        push_batch<NT>(A.G, sm, x, ok, ok ? (long long)Sg[x] : 0ll, act);
-                    });
-                    __syncthreads();
-                    for (int b = 0; b < min(sm.nbig, kBigCap); ++b) {
-                        const int x = sm.big[b];
-                        const int64_t rs = A.G.row[x];
-                        const int d = A.G.deg[x];
-                        const long long s = Sg[x];
-                        for (int s0 = threadIdx.x; s0 < d; s0 += 4 * NT) {
-                            int k[4];
-#pragma unroll
-                            for (int u = 0; u < 4; ++u) k[u] = s0 + NT * u < d ? A.G.col[rs + s0 + NT * u] : -1;
-                            act(s, k);
+                            for (int u = 0; u < kLaneSlots; ++u)
+                                if ((first >> u) & 1u) atomicOr(&N[k[u] >> 5], 1u << (k[u] & 31));
+                            return;
                         }
-                    }
-                } else {
-                    scanned += rest;
-                    held = false;
-                    for (int i = threadIdx.x; i < nw; i += NT) B[i] = 0u;
-                    __syncthreads();
-                    for (int i = lo + threadIdx.x; i < hi; i += NT) atomicOr(&B[qd[i] >> 5], 1u << (qd[i] & 31));
-                    __syncthreads();
-                    auto test = [&](int k) { return bit_of(B, k); };
-                    auto val = [&](int k) { return (long long)Sg[k]; };
-                    auto done = [&](int x, long long sum, bool hit) {
-                        if (hit) {
-                            D[x] = L + 1;
-                            Sg[x] = sum;
-                        }
-                        warp_append(&sm.tail, qd, x, hit);
-                    };
-                    unset_tasks<NT>(sm, V, nw, [&](int x, bool ok) {
-                        pull_batch<NT, long long>(A.G, sm, x, ok, test, val, done);
-                    });
-                    __syncthreads();
-                    const int nb = min(sm.nbig, kBigCap);
-                    for (int b = 0; b < nb; ++b) {
-                        const int x = sm.big[b];
-                        const int64_t rs = A.G.row[x];
-                        const int d = A.G.deg[x];
-                        long long s = 0;
-                        bool h = false;
-                        for (int s0 = threadIdx.x; s0 < d; s0 += NT) {
-                            const int k = A.G.col[rs + s0];
-                            if (test(k)) {
-                                s += val(k);
-                                h = true;
+                        if (first) {
+                            unsigned old[kLaneSlots];
+#pragma unroll
+                            for (int u = 0; u < kLaneSlots; ++u)
+                                old[u] = (first >> u) & 1u ? atomicOr(&N[k[u] >> 5], 1u << (k[u] & 31)) : ~0u;
+#pragma unroll
+                            for (int u = 0; u < kLaneSlots; ++u) {
+                                if ((old[u] >> (k[u] & 31)) & 1u) first &= ~(1u << u);
+                                if ((first >> u) & 1u) D[k[u]] = L + 1;
                             }
                         }
-                        if (h) {
-                            atomic_add_i64(&Sg[x], s);
-                            sm.bighit[b] = 1;
+                        append_first(sm, qd, k, first);
+                    };
+                    list_tasks<NT, long long>(A.G, sm, qd + lo, hi - lo, front, [&](int x) { return (long long)Sg[x]; },
+                                              [&](const TaskVertex<long long>& q, bool) { push_batch(A.G, sm, q, act); });
+                    big_segments(A.G, sm, [&](int, int x, int64_t rs, int s0, int s1) {
+                        const long long s = Sg[x];
+                        for (int i = s0 + lane; i < s1; i += 32 * kLaneSlots) {
+                            int k[kLaneSlots];
+                            load_slots(A.G, rs, s1, i, 32, k);
+                            act(s, k);
                         }
+                        __syncwarp();
+                    });
+                } else {
+                    scanned += rest;
+                    if (MODE == kOneBits && held) {
+                        for (int i = threadIdx.x; i < nw; i += NT) B[i] = 0u;
+                        held = false;
+                        __syncthreads();
                     }
+                    for (int i = lo + threadIdx.x; i < hi; i += NT) atomicOr(&B[qd[i] >> 5], 1u << (qd[i] & 31));
+                    __syncthreads();
+                    auto done = [&](int x, int64_t sum, bool hit) {
+                        if (hit) Sg[x] = sum;
+                        if (hit) atomicOr(&N[x >> 5], 1u << (x & 31));
+                    };
+                    unset_tasks<NT>(A.G, sm, V, nw, [&](const TaskVertex<int>& q, bool ok) {
+                        pull_batch<int64_t>(A.G, sm, q, ok, B, Sg, done);
+                    });
+                    const int nb = big_segments(A.G, sm, [&](int b, int x, int64_t rs, int s0, int s1) {
+                        int64_t s = 0;
+                        unsigned any = 0;
+                        for (int i = s0 + lane; i < s1; i += 32 * kLaneSlots) {
+                            int k[kLaneSlots];
+                            load_slots(A.G, rs, s1, i, 32, k);
+                            any |= sum_in(B, Sg, k, s);
+                        }
+                        if (__any_sync(full, any)) {
+#pragma unroll
+                            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(full, s, o);
+                            if (lane == 0) {
+                                atomic_add_i64(&Sg[x], s);
+                                sm.bighit[b] = 1;
+                            }
+                        }
+                    });
                     if (nb > 0) {
                         __syncthreads();
                         for (int b = threadIdx.x; b < nb; b += NT)
-                            done(sm.big[b], (long long)Sg[sm.big[b]], sm.bighit[b] != 0);
+                            done(sm.big[b], Sg[sm.big[b]], sm.bighit[b] != 0);
                     }
                 }
                 __syncthreads();
+                // B and N are empty again between levels (or B is the visited set)
+                if (pull)
+                    for (int i = lo + threadIdx.x; i < hi; i += NT) B[qd[i] >> 5] = 0u;
+                unsigned long long sum = 0;
                 lo = hi;
-                hi = sm.tail;
+                if (dense) {
+                    // N listed in vertex order, added to the visited set and
+                    // emptied: a warp per run of words
+                    const int run = ((nw + NT / 32 - 1) / (NT / 32) + 31) & ~31;
+                    const int w0 = min(nw, (int)(threadIdx.x >> 5) * run), w1 = min(nw, w0 + run);
+                    int c = 0;
+                    for (int i = w0 + lane; i < w1; i += 32) c += __popc(N[i]);
+                    c = __reduce_add_sync(full, c);
+                    if (lane == 0) sm.wsum[threadIdx.x >> 5] = c;
+                    __syncthreads();
+                    const int mine = lane < NT / 32 ? sm.wsum[lane] : 0;
+                    int pos = lo + __reduce_add_sync(full, lane < (int)(threadIdx.x >> 5) ? mine : 0);
+                    hi = lo + __reduce_add_sync(full, mine);
+                    for (int i0 = w0; i0 < w1 && c; i0 += 32) {
+                        const int i = i0 + lane;
+                        const unsigned word = i < w1 ? N[i] : 0u;
+                        if (word) {
+                            N[i] = 0u;
+                            V[i] |= word;
+                            if (MODE == kOneBits && held) B[i] |= word;
+                        }
+                        for (unsigned have = __ballot_sync(full, word != 0u); have; have &= have - 1) {
+                            const int j = __ffs(have) - 1;
+                            const unsigned w = __shfl_sync(full, word, j);
+                            if ((w >> lane) & 1u) {
+                                const int x = (i0 + j) * 32 + lane;
+                                qd[pos + __popc(w & ((1u << lane) - 1u))] = x;
+                                D[x] = L + 1;
+                                sum += (unsigned)A.G.deg[x];
+                            }
+                            pos += __popc(w);
+                        }
+                    }
+                    if (threadIdx.x == 0) sm.tail = hi;
+                } else {
+                    hi = sm.tail;
+                    for (int i = lo + threadIdx.x; i < hi; i += NT) {
+                        const int x = qd[i];
+                        const unsigned bit = 1u << (x & 31);
+                        atomicOr(&V[x >> 5], bit);
+                        if (MODE == kOneBits && held) atomicOr(&B[x >> 5], bit);
+                        N[x >> 5] = 0u;
+                        sum += (unsigned)A.G.deg[x];
+                    }
+                }
                 if (lo == hi) break;
                 ++L;
-                unsigned long long sum = 0;
-                for (int i = lo + threadIdx.x; i < hi; i += NT) {
-                    const int x = qd[i];
-                    const unsigned bit = 1u << (x & 31);
-                    atomicOr(&V[x >> 5], bit);
-                    if (MODE == kOneBits && held) atomicOr(&B[x >> 5], bit);
-                    sum += (unsigned)A.G.deg[x];
-                }
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(full, sum, o);
                 if (lane == 0 && sum) atomicAdd(&sm.slots, sum);
@@ -536,12 +778,13 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
 
             // ---- backward: each vertex sums its children's weights
             // w = (delta + 1) / sigma, kept in acc ----
-            for (int i = threadIdx.x; i < nw; i += NT) B[i] = 0u;
+            if (MODE == kOneBits && held)
+                for (int i = threadIdx.x; i < nw; i += NT) B[i] = 0u;
             auto finish = [&](int x, double sum) {
-                const double sx = (double)Sg[x];
-                const double nd = sx * sum;
+                const int64_t sg = Sg[x];
+                const double nd = (double)sg * sum;
                 Dl[x] = nd;
-                acc[x] = (nd + 1.0) / sx;
+                acc[x] = child_weight(nd + 1.0, sg);
             };
             for (int i = lvl[nlev - 1] + threadIdx.x; i < reached; i += NT) finish(qd[i], 0.0);
             __syncthreads();
@@ -557,54 +800,46 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                 }
                 __syncthreads();
                 if (push) {
-                    auto act = [&](double w, const int (&k)[4]) {
+                    auto act = [&](double w, const int (&k)[kLaneSlots]) {
+                        const unsigned in = in_bitmap(B, k);
 #pragma unroll
-                        for (int u = 0; u < 4; ++u)
-                            if (k[u] >= 0 && bit_of(B, k[u])) atomicAdd(&acc[k[u]], w);
+                        for (int u = 0; u < kLaneSlots; ++u)
+                            if ((in >> u) & 1u) atomicAdd(&acc[k[u]], w);
                     };
-                    list_tasks<NT>(sm, qd + a1, end - a1, [&](int x, bool ok) {
-                        push_batch<NT>(A.G, sm, x, ok, ok ? acc[x] : 0.0, act);
-                    });
-                    __syncthreads();
-                    const int nb = min(sm.nbig, kBigCap);
-                    for (int b = 0; b < nb; ++b) {
-                        const int x = sm.big[b];
-                        const int64_t rs = A.G.row[x];
-                        const int d = A.G.deg[x];
+                    list_tasks<NT, double>(A.G, sm, qd + a1, end - a1, sm.lvslots[l + 1], [&](int x) { return acc[x]; },
+                                           [&](const TaskVertex<double>& q, bool) { push_batch(A.G, sm, q, act); });
+                    const int nb = big_segments(A.G, sm, [&](int, int x, int64_t rs, int s0, int s1) {
                         const double w = acc[x];
-                        for (int s0 = threadIdx.x; s0 < d; s0 += 4 * NT) {
-                            int k[4];
-#pragma unroll
-                            for (int u = 0; u < 4; ++u) k[u] = s0 + NT * u < d ? A.G.col[rs + s0 + NT * u] : -1;
+                        for (int i = s0 + lane; i < s1; i += 32 * kLaneSlots) {
+                            int k[kLaneSlots];
+                            load_slots(A.G, rs, s1, i, 32, k);
                             act(w, k);
                         }
-                    }
+                        __syncwarp();
+                    });
                     if (nb > 0) __syncthreads();
                     for (int i = a0 + threadIdx.x; i < a1; i += NT) finish(qd[i], acc[qd[i]]);
                 } else {
-                    auto test = [&](int k) { return bit_of(B, k); };
-                    auto val = [&](int k) { return acc[k]; };
-                    list_tasks<NT>(sm, qd + a0, a1 - a0, [&](int x, bool ok) {
-                        pull_batch<NT, double>(A.G, sm, x, ok, test, val,
-                                               [&](int y, double sum, bool) { finish(y, sum); });
-                    });
-                    __syncthreads();
-                    const int nb = min(sm.nbig, kBigCap);
-                    for (int b = 0; b < nb; ++b) {
-                        const int x = sm.big[b];
-                        const int64_t rs = A.G.row[x];
-                        const int d = A.G.deg[x];
+                    list_tasks<NT, int>(A.G, sm, qd + a0, a1 - a0, l < kSlotLevels ? sm.lvslots[l] : 0ull,
+                                        [](int) { return 0; },
+                                        [&](const TaskVertex<int>& q, bool ok) {
+                                            pull_batch<double>(A.G, sm, q, ok, B, acc,
+                                                                   [&](int y, double sum, bool) { finish(y, sum); });
+                                        });
+                    const int nb = big_segments(A.G, sm, [&](int, int x, int64_t rs, int s0, int s1) {
                         double s = 0.0;
-                        for (int s0 = threadIdx.x; s0 < d; s0 += NT) {
-                            const int k = A.G.col[rs + s0];
-                            if (test(k)) s += val(k);
+                        unsigned any = 0;
+                        for (int i = s0 + lane; i < s1; i += 32 * kLaneSlots) {
+                            int k[kLaneSlots];
+                            load_slots(A.G, rs, s1, i, 32, k);
+                            any |= sum_in(B, acc, k, s);
                         }
-                        if (__any_sync(full, s != 0.0)) {
+                        if (__any_sync(full, any)) {
 #pragma unroll
                             for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(full, s, o);
                             if (lane == 0) atomicAdd(&acc[x], s);
                         }
-                    }
+                    });
                     if (nb > 0) {
                         __syncthreads();
                         for (int b = threadIdx.x; b < nb; b += NT) finish(sm.big[b], acc[sm.big[b]]);
@@ -691,23 +926,26 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
 }
 
 // bc[v] = sum over roots r of delta[r][v], skipping v == root.  A block takes
-// kSumCols vertices at a time and shares the roots out among kSumParts rows of
-// threads (each in root order; the parts are added in order at the end): with a
-// thread per vertex alone, a graph of 1,024 vertices summed its 1,024 roots on
-// four blocks.
-constexpr int kSumCols = 32, kSumParts = 16;
+// COLS vertices at a time and shares the roots out among its rows of threads
+// (each in root order; the rows are added in order at the end).  Large graphs
+// are bound by the fp64 adds (R-MAT 20, 1,024 roots: 2.1 ms, 1.07 G adds at
+// about 3 per ns and SM); on small ones the time is the chain of loads per
+// thread, so few columns and more rows (ER 1,024, 1,024 roots: 20 us with 32
+// columns, 258 us with a thread per vertex).
+constexpr int kSumThreads = 512;
 
-__global__ void __launch_bounds__(kSumCols* kSumParts) k_bc_colsum(const double* __restrict__ delta,
-                                                                   const int64_t* __restrict__ roots, int nk,
-                                                                   int64_t nv, double* __restrict__ bc,
-                                                                   const int* __restrict__ abort)
+template <int COLS>
+__global__ void __launch_bounds__(kSumThreads) k_bc_colsum(const double* __restrict__ delta,
+                                                           const int64_t* __restrict__ roots, int nk, int64_t nv,
+                                                           double* __restrict__ bc, const int* __restrict__ abort)
 {
-    __shared__ double part[kSumParts][kSumCols];
+    constexpr int PARTS = kSumThreads / COLS;
+    __shared__ double part[PARTS][COLS];
     if (abort && *abort) return;
-    const int c = threadIdx.x % kSumCols, p = threadIdx.x / kSumCols;
-    const int per = (nk + kSumParts - 1) / kSumParts;
+    const int c = threadIdx.x % COLS, p = threadIdx.x / COLS;
+    const int per = (nk + PARTS - 1) / PARTS;
     const int r0 = min(nk, p * per), r1 = min(nk, r0 + per);
-    for (int64_t v0 = blockIdx.x * (int64_t)kSumCols; v0 < nv; v0 += (int64_t)gridDim.x * kSumCols) {
+    for (int64_t v0 = blockIdx.x * (int64_t)COLS; v0 < nv; v0 += (int64_t)gridDim.x * COLS) {
         const int64_t v = v0 + c;
         double s = 0.0;
         if (v < nv) {
@@ -720,11 +958,23 @@ __global__ void __launch_bounds__(kSumCols* kSumParts) k_bc_colsum(const double*
         part[p][c] = s;
         __syncthreads();
         if (p == 0 && v < nv) {
-            for (int q = 1; q < kSumParts; ++q) s += part[q][c];
+            for (int q = 1; q < PARTS; ++q) s += part[q][c];
             bc[v] = s;
         }
         __syncthreads();
     }
+}
+
+// 32 columns read whole lines; below about 8,192 vertices 8 columns give the
+// SMs four times the blocks.
+cudaError_t launch_bc_colsum(const double* delta, const int64_t* roots, int nk, int64_t nv, double* bc,
+                             const int* abort, cudaStream_t s)
+{
+    const int cols = nv <= 8192 ? 8 : 32;
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((nv + cols - 1) / cols, 8192));
+    if (cols == 8) k_bc_colsum<8><<<grid, kSumThreads, 0, s>>>(delta, roots, nk, nv, bc, abort);
+    else k_bc_colsum<32><<<grid, kSumThreads, 0, s>>>(delta, roots, nk, nv, bc, abort);
+    return cudaGetLastError();
 }
 
 // Two-bit rows (dist mod 3, 3 = unreachable; 16 vertices per word) of every
@@ -766,16 +1016,22 @@ struct StaticShape {
     StaticKernel kernel;
 };
 
-size_t static_dyn(int mode, int64_t nv)
+size_t static_dyn(int mode, int64_t nv, bool third)
 {
     const size_t nw = (size_t)((nv + 31) / 32) * 4;
-    return mode == kSmall ? (size_t)nv * 28 + 2 * nw : mode == kBits ? 2 * nw : mode == kOneBits ? nw : 0;
+    return mode == kSmall ? (size_t)nv * 28 + 3 * nw : mode == kBits ? (third ? 3 : 2) * nw : mode == kOneBits ? nw : 0;
 }
 
-size_t static_fixed(int nt)
+template <int CAP>
+size_t static_fixed_cap(int nt)
 {
-    return nt == 128 ? sizeof(StaticSmem<128>) : nt == 256 ? sizeof(StaticSmem<256>)
-         : nt == 512 ? sizeof(StaticSmem<512>) : sizeof(StaticSmem<1024>);
+    return nt == 128 ? sizeof(StaticSmem<128, CAP>) : nt == 256 ? sizeof(StaticSmem<256, CAP>)
+         : nt == 512 ? sizeof(StaticSmem<512, CAP>) : sizeof(StaticSmem<1024, CAP>);
+}
+
+size_t static_fixed(int nt, int mode)
+{
+    return mode == kSmall ? static_fixed_cap<kBigCapSmall>(nt) : static_fixed_cap<kBigCap>(nt);
 }
 
 StaticKernel static_kernel(int nt, int mode)
@@ -800,21 +1056,21 @@ int pow2_floor(int64_t x)
 // there are roots for (1,024 threads per SM are shared out among them: the
 // kernel takes up to 64 registers per thread), as the shared memory holds and,
 // where the rows' scratch is in HBM, as there are scratch slots; an update
-// worker's scratch has room for two static workers where both bitmaps are in
-// shared memory.
+// worker's scratch has room for two static workers where the bitmaps are in
+// shared memory.  hbm_bits: the scratch has room for bitmaps.
 StaticShape static_shape(int64_t nv, int64_t nk, int64_t workers, int sm_count, size_t smem_block, size_t smem_sm,
-                         bool may_halve)
+                         bool hbm_bits)
 {
     StaticShape S;
     S.mode = kSmall;
-    while (S.mode != kNoBits && static_dyn(S.mode, nv) + static_fixed(1024) + 1024 > smem_block) ++S.mode;
-    S.dyn = static_dyn(S.mode, nv);
-    S.halves = S.mode == kBits && may_halve ? 2 : 1;
+    while (S.mode != kNoBits && static_dyn(S.mode, nv, !hbm_bits) + static_fixed(1024, S.mode) + 1024 > smem_block) ++S.mode;
+    S.dyn = static_dyn(S.mode, nv, !hbm_bits);
+    S.halves = S.mode == kBits && hbm_bits ? 2 : 1;
     int64_t c = std::max<int64_t>(1, (nk + sm_count - 1) / sm_count);
     c = std::min<int64_t>(c, S.mode == kSmall ? 8 : S.mode == kBits ? 4 : 1);
     if (S.mode != kSmall) c = std::min<int64_t>(c, std::max<int64_t>(1, (workers * S.halves + sm_count - 1) / sm_count));
     // fewer CTAs while the SM's shared memory does not hold them (1 KB each is the system's)
-    while (c > 1 && (size_t)c * (S.dyn + static_fixed(pow2_floor(1024 / c)) + 1024) > smem_sm) --c;
+    while (c > 1 && (size_t)c * (S.dyn + static_fixed(pow2_floor(1024 / c), S.mode) + 1024) > smem_sm) --c;
     S.nt = std::max(pow2_floor(1024 / c), S.mode == kSmall ? 128 : S.mode == kBits ? 256 : 1024);
     S.grid = (int)std::min<int64_t>(nk, c * sm_count);
     if (S.mode != kSmall) S.grid = (int)std::min<int64_t>(S.grid, workers * S.halves);
@@ -824,7 +1080,7 @@ StaticShape static_shape(int64_t nv, int64_t nk, int64_t workers, int sm_count, 
 
 cudaError_t static_launch(const StaticShape& S, const StaticArgs& A, cudaStream_t s)
 {
-    if (S.dyn + static_fixed(S.nt) > 48 * 1024) {
+    if (S.dyn + static_fixed(S.nt, S.mode) > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(S.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.dyn);
         if (e) return e;
     }
@@ -880,15 +1136,13 @@ cudaError_t launch_static_list(sbc_forest* f, const int* d_list, const int* d_nl
     A.asym_dev = nullptr;
     const StaticShape S = static_shape(f->nv, n, f->workers, f->sm_count, smem_block, smem_sm, true);
     A.halves = S.halves;
+    A.third_bits = 0;
     f->prof_begin(PROF_STATIC);
     e = static_launch(S, A, s);
     f->prof_end(PROF_STATIC);
     if (e) return e;
     if (d_list) return cudaSuccess;  // the caller moves BC by the listed roots' old and new rows
-    const int bgrid = (int)std::min<int64_t>((f->nv + kSumCols - 1) / kSumCols, (int64_t)f->sm_count * 64);
-    k_bc_colsum<<<std::max(bgrid, 1), kSumCols * kSumParts, 0, s>>>(f->d_delta, f->d_roots, (int)f->nk, f->nv,
-                                                                    f->d_bc, nullptr);
-    return cudaGetLastError();
+    return launch_bc_colsum(f->d_delta, f->d_roots, (int)f->nk, f->nv, f->d_bc, nullptr, s);
 }
 
 }  // namespace sbc
@@ -1097,10 +1351,11 @@ extern "C" int sbc_static_init_noalloc(int64_t nv, const int64_t* d_off, const i
     const StaticShape S = static_shape(nv, slots, slots, slots, smem_block, smem_sm, false);
     if (S.mode > kBits) return noalloc_fail(SBC_ERR_CUDA, "sbc_static_init_noalloc: too little shared memory");
     A.halves = 1;
-    if (static_launch(S, A, s) != cudaSuccess) return noalloc_fail(SBC_ERR_CUDA, "sbc_static_init_noalloc: k_static launch failed");
-    const int bgrid = (int)std::min<int64_t>((nv + kSumCols - 1) / kSumCols, 8192);
-    k_bc_colsum<<<bgrid, kSumCols * kSumParts, 0, s>>>(d_delta, d_roots, (int)nk, nv, d_bc, bad);
-    if (noalloc_launch_failed("k_bc_colsum", &rc)) return rc;
+    A.third_bits = S.mode == kBits;
+    if (static_launch(S, A, s) != cudaSuccess)
+        return noalloc_fail(SBC_ERR_CUDA, "sbc_static_init_noalloc: k_static launch failed");
+    if (launch_bc_colsum(d_delta, d_roots, (int)nk, nv, d_bc, bad, s) != cudaSuccess)
+        return noalloc_fail(SBC_ERR_CUDA, "sbc_static_init_noalloc: k_bc_colsum launch failed");
     // wait for the work and read the input-check word (a 4-byte copy into a
     // stack variable: no allocation)
     int h_bad = 0;

@@ -36,8 +36,8 @@ def _mixed(nv, seed):
     return g, np.asarray(roots, dtype=np.int64)
 
 
-# around the largest graph whose rows fit in shared memory (about 7,860 vertices), and the sizes of which two bitmaps
-# (about 0.89 million) or one (1.78 million) do
+# around the largest graph whose rows fit in shared memory (about 7,860 vertices), and the sizes of which two
+# bitmaps (about 0.89 million) or one (1.77 million) do
 @pytest.mark.parametrize("nv", [2, 31, 33, 200, 1025, 4100, 7800, 7900, 45001, 300007, 1000003, 1800001])
 def test_static_at_every_size_class(sbc_lib, port_lib, nv):
     g, roots = _mixed(nv, seed=nv)
