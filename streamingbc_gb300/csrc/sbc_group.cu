@@ -35,12 +35,13 @@ struct GroupUpdateArgs {
     unsigned long long* counters;
 };
 
-// One thread per (member, root): the pair joins the batch's worklist iff some
-// live insertion of that member's batch joins two different levels of the
-// root's tree (as k_classify does for one forest).
+// One warp per (member, root), lanes over that member's insertions: the pair
+// joins the batch's worklist iff some live insertion joins two different levels
+// of the root's tree (as k_classify does for one forest).
 __global__ void k_classify_group(const __grid_constant__ GroupUpdateArgs A)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
+    const int lane = threadIdx.x & 31;
     if (i >= A.root_base[A.nslots]) return;
     int lo = 0, hi = A.nslots - 1;
     while (lo < hi) {
@@ -52,9 +53,11 @@ __global__ void k_classify_group(const __grid_constant__ GroupUpdateArgs A)
     const int r = i - A.root_base[lo];
     const int32_t* D = P.dist + (size_t)r * P.G.nv;
     bool active = false;
-    for (int k = 0; k < P.nins && !active; ++k)
-        if (P.ins_ok[k] > 0 && D[P.ins_u[k]] != D[P.ins_v[k]]) active = true;
-    if (active) A.worklist[atomicAdd(A.nwork, 1)] = ((uint32_t)lo << kSlotShift) | (uint32_t)r;
+    for (int base = 0; base < P.nins && !active; base += 32) {
+        const int k = base + lane;
+        active = __any_sync(0xffffffffu, k < P.nins && P.ins_ok[k] > 0 && D[P.ins_u[k]] != D[P.ins_v[k]]);
+    }
+    if (lane == 0 && active) A.worklist[atomicAdd(A.nwork, 1)] = ((uint32_t)lo << kSlotShift) | (uint32_t)r;
 }
 
 template <int NT, int MINB, int ILP>
@@ -146,7 +149,7 @@ cudaError_t launch_group_update(sbc_group* G, const int* counts, unsigned steps)
     if (steps & GROUP_UPDATE) {
         if ((e = cudaMemsetAsync(G->d_nwork, 0, 2 * sizeof(int), s))) return e;
         const int total = A.root_base[ns];
-        k_classify_group<<<(total + 255) / 256, 256, 0, s>>>(A);
+        k_classify_group<<<(int)(((int64_t)total * 32 + 127) / 128), 128, 0, s>>>(A);
         if ((e = cudaGetLastError())) return e;
         const int grid = (int)std::min<int64_t>(G->ws.workers, total);
         kGroupVariants[G->variant].launch(A, grid, s);

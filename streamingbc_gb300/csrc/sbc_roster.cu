@@ -17,8 +17,9 @@
 // k_roster_compact drops stale entries after each batch.
 //   k_roster_build    CTA per root: members of levels 2..kRosterLevels-1 whose
 //                     level histogram count fits a roster (after static init)
-//   k_roster_compact  warp per (root, level) roster marked stale (the _group
-//                     form: for several forests in one launch)
+//   k_roster_compact  thread per (root, level) roster, the warp together for
+//                     each one marked stale (the _group form: for several
+//                     forests in one launch)
 #include "sbc_host.h"
 #include "sbc_internal.cuh"
 
@@ -56,12 +57,12 @@ __global__ void __launch_bounds__(256) k_roster_build(const uint8_t* __restrict_
     }
 }
 
-// Warp w = root * kRosterLevels + level drops the stale entries of its roster.
+// The calling warp drops the stale entries of roster w = root * kRosterLevels +
+// level.
 __device__ __forceinline__ void compact_one(const uint8_t* __restrict__ dist8, int64_t nv,
                                             int32_t* __restrict__ roster, int32_t* __restrict__ roster_n,
                                             int32_t* __restrict__ dirty, int w, int lane)
 {
-    if (!dirty[w]) return;  // warp-uniform
     const int n = roster_n[w];
     if (n > kRosterCap) return;
     const int level = w % kRosterLevels;
@@ -88,9 +89,11 @@ __global__ void __launch_bounds__(256) k_roster_compact(const uint8_t* __restric
                                                         int32_t* __restrict__ roster, int32_t* __restrict__ roster_n,
                                                         int32_t* __restrict__ dirty)
 {
-    const int w = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
-    if (w >= nk * kRosterLevels) return;
-    compact_one(dist8, nv, roster, roster_n, dirty, w, threadIdx.x & 31);
+    // a lane looks at each roster's flag; the warp takes the marked ones together
+    const int w = (int)(blockIdx.x * (size_t)blockDim.x + threadIdx.x);
+    const int lane = threadIdx.x & 31;
+    for (unsigned m = __ballot_sync(0xffffffffu, w < nk * kRosterLevels && dirty[w]); m; m &= m - 1)
+        compact_one(dist8, nv, roster, roster_n, dirty, w - lane + __ffs(m) - 1, lane);
 }
 
 // Several forests in one launch (the members of a group batch).
@@ -110,16 +113,22 @@ struct RosterGroupArgs {
 
 __global__ void __launch_bounds__(256) k_roster_compact_group(const __grid_constant__ RosterGroupArgs A)
 {
-    const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    if (w >= A.wbase[A.nf]) return;
+    const int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
     int lo = 0, hi = A.nf - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (A.wbase[mid] <= w) lo = mid;
         else hi = mid - 1;
     }
-    const RosterForest& F = A.f[lo];
-    compact_one(F.dist8, F.nv, F.roster, F.roster_n, F.dirty, (int)(w - A.wbase[lo]), threadIdx.x & 31);
+    const bool marked = w < A.wbase[A.nf] && A.f[lo].dirty[w - A.wbase[lo]];
+    for (unsigned m = __ballot_sync(0xffffffffu, marked); m; m &= m - 1) {
+        const int j = __ffs(m) - 1;
+        const int64_t wj = w - lane + j;
+        const RosterForest& F = A.f[__shfl_sync(0xffffffffu, lo, j)];
+        compact_one(F.dist8, F.nv, F.roster, F.roster_n, F.dirty,
+                    (int)(wj - A.wbase[__shfl_sync(0xffffffffu, lo, j)]), lane);
+    }
 }
 
 cudaError_t launch_roster_compact_forests(sbc_forest* const* fs, int nf, cudaStream_t s)
@@ -141,7 +150,7 @@ cudaError_t launch_roster_compact_forests(sbc_forest* const* fs, int nf, cudaStr
             ++A.nf;
         }
         if (A.nf == 0) continue;
-        k_roster_compact_group<<<(int)((A.wbase[A.nf] * 32 + 255) / 256), 256, 0, s>>>(A);
+        k_roster_compact_group<<<(int)((A.wbase[A.nf] + 255) / 256), 256, 0, s>>>(A);
         cudaError_t e = cudaGetLastError();
         if (e) return e;
     }
@@ -161,8 +170,8 @@ cudaError_t launch_roster_build_list(sbc_forest* f, const int* d_list, const int
 cudaError_t launch_roster_compact(sbc_forest* f, cudaStream_t s)
 {
     if (!f->d_roster) return cudaSuccess;
-    const int64_t warps = f->nk * kRosterLevels;
-    k_roster_compact<<<(int)((warps * 32 + 255) / 256), 256, 0, s>>>(
+    const int64_t rosters = f->nk * kRosterLevels;
+    k_roster_compact<<<(int)((rosters + 255) / 256), 256, 0, s>>>(
         f->d_dist8, f->nv, (int)f->nk, f->d_roster, f->d_roster_n, f->d_roster_dirty);
     return cudaGetLastError();
 }
