@@ -76,3 +76,35 @@ def test_deletions_from_an_unsorted_tail(sbc_lib, port_lib):
     _check(f, G.delete_edges(G.insert_edges(g, ins), dels), roots, port_lib)
     f.close()
     dg.close()
+
+
+@pytest.mark.parametrize("nv,m,call", [(300, 900, 5), (300, 900, 40), (2000, 5000, 16)])
+def test_level2_masks_follow_deletions(sbc_lib, port_lib, nv, m, call):
+    """Deletions around the roots' neighbours (edges of a root, of its neighbours, between two of them, and others),
+    many in one call, with roots of few and of more than 32 neighbours; then insertions that rely on the masks."""
+    rng = np.random.default_rng(nv + call)
+    g = G.er(nv, m, seed=call)
+    hub = np.stack([np.full(50, 4), rng.choice(np.arange(5, nv), 50, replace=False)], 1)
+    g = G.insert_edges(g, hub)
+    roots = np.asarray(sorted({4, *rng.choice(np.arange(5, nv), 11, replace=False).tolist()}))
+    dg = native.DeviceGraph(g.nv, g.off, g.adj)
+    f = native.DeviceForest(dg, roots)
+    f.set_delete_mode(native.DeviceForest.DELETE_MOVE_DOWN)
+    f.static_init()
+    for step in range(3):
+        e = G.edge_list(g)
+        near = np.isin(e, roots).any(1)
+        nb = np.unique(e[near])
+        second = np.isin(e, nb).any(1) & ~near
+        pick = np.concatenate([rng.permutation(e[near])[:call // 5 + 1], rng.permutation(e[second])[:call],
+                               rng.permutation(e)[:call // 3 + 1]])
+        pick = rng.permutation(np.unique(pick, axis=0))[:call]
+        assert f.delete(pick)["inserted"] == len(pick)
+        g = G.delete_edges(g, pick)
+        _check(f, g, roots, port_lib)
+        ins = G.uniform_insertions(g, 8, seed=step)
+        assert f.insert(ins)["inserted"] == 8
+        g = G.insert_edges(g, ins)
+        _check(f, g, roots, port_lib)
+    f.close()
+    dg.close()
