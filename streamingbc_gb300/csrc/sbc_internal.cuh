@@ -543,6 +543,38 @@ __device__ __forceinline__ void lb_walk_sum(const DevGraph& G, int g, const Dist
     }
 }
 
+// Child weights (delta + 1) / sigma.  An SM issues one fp64 instruction per 16
+// cycles, each waiting for the one before, and the compiler's division is the
+// longest chain of them in a commit.  Here the reciprocal of sigma starts from
+// the fp32 one (24 bits), one Newton step doubles its bits, and the quotient's
+// remainder, exact by fused multiply-add, corrects the quotient to the last bit
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990): five fp64 instructions, three where the reciprocal is at
+// hand.
+struct Sigma {
+    double b, r;  // its value and its reciprocal to about 46 bits (0: divide plainly)
+};
+
+__device__ __forceinline__ Sigma sigma_of(int64_t s)
+{
+    Sigma q{(double)s, 0.0};
+    if (s > 0) {  // a sum that wrapped may be 0 or negative
+        const int f = __float_as_int(__frcp_rn(__ll2float_rn(s)));
+        // the float's value as a double
+        const double r0 = __hiloint2double((f >> 3) + (896 << 20), (int)((unsigned)f << 29));
+        q.r = fma(r0, fma(-q.b, r0, 1.0), r0);
+    }
+    return q;
+}
+
+__device__ __forceinline__ double child_weight(double a, const Sigma& s)
+{
+    // values that are not finite: plain division
+    if (__double2hiint(s.r) == 0 || ((unsigned)__double2hiint(a) & 0x7fffffffu) >= 0x7fd00000u) return a / s.b;
+    const double q = a * s.r;
+    return fma(fma(-s.b, q, a), s.r, q);
+}
+
 // Block-wide sums of two 64-bit integers and one double per thread; every
 // thread gets the three totals.  Warps reduce with shuffles, then warp 0 adds
 // the per-warp partials and publishes the totals.  GB300 issues fp64 at a

@@ -164,24 +164,6 @@ __device__ __forceinline__ void add_shared(int64_t* p, long long v)
     if (hi) atomicAdd((unsigned*)p + 1, hi);
 }
 
-// a / s.  The SM issues one fp64 instruction per 16 cycles, and a division by
-// the compiler takes more of them than all else done per vertex: here the
-// reciprocal starts from the fp32 one (24 bits), one Newton step doubles its
-// bits, and the quotient's remainder, exact by fused multiply-add, corrects the
-// quotient to the last bit (Markstein, "Computation of elementary functions on
-// the IBM RISC System/6000 processor", 1990): five fp64 instructions.
-__device__ __forceinline__ double child_weight(double a, int64_t s)
-{
-    const double b = (double)s;
-    // s <= 0 (a sum that wrapped) and values that are not finite: plain division
-    if (s <= 0 || (unsigned)__double2hiint(a) >= 0x7fd00000u) return a / b;
-    const int f = __float_as_int(__frcp_rn(__ll2float_rn(s)));
-    const double r = __hiloint2double((f >> 3) + (896 << 20), f << 29);  // the float's value
-    const double r1 = fma(r, fma(-b, r, 1.0), r);
-    const double q = a * r1;
-    return fma(fma(-b, q, a), r1, q);
-}
-
 // A vertex held by one lane of a task: its slots and its value.
 template <class V>
 struct TaskVertex {
@@ -781,10 +763,10 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
             if (MODE == kOneBits && held)
                 for (int i = threadIdx.x; i < nw; i += NT) B[i] = 0u;
             auto finish = [&](int x, double sum) {
-                const int64_t sg = Sg[x];
-                const double nd = (double)sg * sum;
+                const Sigma sw = sigma_of(Sg[x]);
+                const double nd = sw.b * sum;
                 Dl[x] = nd;
-                acc[x] = child_weight(nd + 1.0, sg);
+                acc[x] = child_weight(nd + 1.0, sw);
             };
             for (int i = lvl[nlev - 1] + threadIdx.x; i < reached; i += NT) finish(qd[i], 0.0);
             __syncthreads();

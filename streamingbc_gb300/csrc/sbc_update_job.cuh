@@ -149,7 +149,7 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
     int64_t* S = A.sigma + (size_t)r * nv;
     double* Dl = A.delta + (size_t)r * nv;
     const int root = (int)A.roots[r];
-    const int aL = DECR ? D[a] : 0;
+    const int aL = DECR || del ? D[a] : 0;
 
     // ---------------- ascent ----------------
     // A parent k's delta gains, per child x, sigma_k * (newdelta_x+1)/newsigma_x,
@@ -171,18 +171,16 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
         const double oD = Dl[x];
         const double ac = W.acc[x];
         const int64_t nS = isDown ? (mv ? W.dp[x] : oS + W.dp[x]) : oS;
-        const double nD = isDown ? (double)nS * ac : oD + (double)oS * ac;
-        wn = (nD + 1.0) / (double)nS;
-        wd = oS ? wn - (oD + 1.0) / (double)oS : wn;
+        const Sigma ws = sigma_of(nS);
+        const double nD = isDown ? ws.b * ac : oD + ws.b * ac;
+        wn = child_weight(nD + 1.0, ws);
+        wd = oS ? wn - child_weight(oD + 1.0, isDown ? sigma_of(oS) : ws) : wn;
         if (x != root) atomicAdd(&A.bc[x], nD - oD);
         S[x] = nS;
         Dl[x] = nD;
-        if (!DECR && del && x == b) {
-            // a (one level up, not in the descent) loses b's old contribution
-            int old = atomicOr(&W.st[a], SBC_ASC);
-            if (!(old & SBC_ASC)) W.qa[atomicAdd(&sm.at, 1)] = a;
-            atomicAdd(&W.acc[a], wd - wn);
-        }
+        // a (one level up, not in the descent) loses b's old contribution; it
+        // is claimed when its level has been walked
+        if (!DECR && del && x == b) atomicAdd(&W.acc[a], wd - wn);
     };
     auto prep = [&](int j, int x, int d) {
         double wn, wd;
@@ -304,9 +302,12 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
     };
     auto probe_diverted = [&]() {
         const int n = sm.nprobe;
-        __syncthreads();
-        if (threadIdx.x == 0) sm.nprobe = 0;
         if (n > 0) probe_parents(W.lvl + nv + 2 - n, n, rcand, rcnt, true);
+        __syncthreads();  // every thread has read the count
+        if (n > 0) {
+            if (threadIdx.x == 0) sm.nprobe = 0;
+            __syncthreads();  // and the next level lists into an empty list
+        }
     };
 
     int ua_lo = 0, ua_hi = 0;
@@ -319,7 +320,7 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
             dlist = W.qd + W.lvl[ds];
             dn = W.lvl[ds + 1] - W.lvl[ds];
         }
-        const int next_lo = sm.at;
+        const int next_lo = ua_hi;  // nothing was claimed since it was read
         const bool pull_ok = L >= 1 && L <= 2 && (!moving || L < Lb);
         rcand = nullptr;
         rcnt = 0;
@@ -332,13 +333,12 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
             }
         }
         if (L == 0) {
-            // The root alone (if reached): no parents, committing is all.
-            if (threadIdx.x == 0 && dn + ua_hi - ua_lo > 0) {
-                const int x = dn ? dlist[0] : W.qa[ua_lo];
-                double wn, wd;
-                commit(x, wn, wd);
+            // The root alone (if reached; a descent never holds it): its
+            // dependency, no weights and no BC.
+            if (threadIdx.x == 0 && ua_hi - ua_lo > 0) {
+                Dl[root] += (double)S[root] * W.acc[root];
                 sm.lb.walked_v += 1;
-                sm.lb.walked_e += (unsigned)vis_deg(A.G, x, A.G.row[x], g);
+                sm.lb.walked_e += (unsigned)vis_deg(A.G, root, A.G.row[root], g);
             }
             __syncthreads();
         } else {
@@ -403,6 +403,9 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
                 const int64_t rrow = A.G.row[root];
                 const int rdeg = vis_deg(A.G, root, rrow, g);
                 const bool rootDown = (W.st[root] & SBC_STEP_MASK) != 0;
+                // the loop below claims (masks) or lists vertices: every thread
+                // has read the counts of the level before
+                if (L == 2) __syncthreads();
                 long long push_cost = 0, mixed_cost = 0;
                 double root_sum = 0.0;
                 const int qbase = sm.st;  // free tail of the same-level queue holds the two lists
@@ -459,18 +462,30 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
                         }
                     }
                 }
-                block_sum3<NT>(push_cost, mixed_cost, root_sum, sm.part);
-                if (threadIdx.x == 0) {
-                    sm.lb.walked_v += (unsigned)(nn1 + nn2);
-                    sm.lb.walked_e += (unsigned long long)push_cost;
-                }
-                if (L == 1) {
-                    if (threadIdx.x == 0 && nn1 + nn2 > 0) {
-                        W.acc[root] += root_sum;
-                        if (!rootDown) {
-                            int old = atomicOr(&W.st[root], SBC_ASC);
-                            if (!(old & SBC_ASC)) W.qa[atomicAdd(&sm.at, 1)] = root;
+                if (L == 2 && !M2) {
+                    block_sum3<NT>(push_cost, mixed_cost, root_sum, sm.part);
+                    if (threadIdx.x == 0) sm.lb.walked_e += (unsigned long long)push_cost;
+                } else {
+                    // a level's few vertices sit in the first warps: each adds
+                    // its own sums, no block reduction
+                    if (__any_sync(0xffffffffu, push_cost != 0)) {
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) push_cost += __shfl_xor_sync(0xffffffffu, push_cost, o);
+                        if (L == 1) {
+#pragma unroll
+                            for (int o = 16; o > 0; o >>= 1) root_sum += __shfl_xor_sync(0xffffffffu, root_sum, o);
                         }
+                        if ((threadIdx.x & 31) == 0) {
+                            atomicAdd(&sm.lb.walked_e, (unsigned long long)push_cost);
+                            if (L == 1) atomicAdd(&W.acc[root], root_sum);
+                        }
+                    }
+                }
+                if (threadIdx.x == 0) sm.lb.walked_v += (unsigned)(nn1 + nn2);
+                if (L == 1) {
+                    if (threadIdx.x == 0 && nn1 + nn2 > 0 && !rootDown) {
+                        int old = atomicOr(&W.st[root], SBC_ASC);
+                        if (!(old & SBC_ASC)) W.qa[atomicAdd(&sm.at, 1)] = root;
                     }
                     __syncthreads();
                 } else if (L == 2 && nn1 + nn2 > 0 && M2) {
@@ -501,8 +516,8 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
                 }
             }
         }
-        if (DECR && L == aL + 1) {
-            // a lost b's old weight (seeded in acc[a]): walked at its level
+        if ((DECR || del) && L == aL + 1) {
+            // a lost b's old weight (in acc[a] already): walked at its level
             if (threadIdx.x == 0) {
                 const int old = atomicOr(&W.st[a], SBC_ASC);
                 if (!(old & SBC_ASC)) W.qa[atomicAdd(&sm.at, 1)] = a;
