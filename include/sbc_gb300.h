@@ -116,7 +116,8 @@ int sbc_graph_create_dimacs(sbc_graph **out, const char *path, int64_t *nv, int6
  * persistent CTAs are sized from occupancy and free memory (0 = automatic). */
 int sbc_forest_create(sbc_forest **out, sbc_graph *g, int64_t nk, const int64_t *roots, int64_t workers);
 /* As sbc_forest_create with an explicit launch shape of the update kernel
- * (variant -1: the SBC_UPDATE_VARIANT environment variable, else the default). */
+ * (variant -1: the SBC_UPDATE_VARIANT environment variable, else by the size of
+ * the graph's adjacency). */
 int sbc_forest_create_ex(sbc_forest **out, sbc_graph *g, int64_t nk, const int64_t *roots, int64_t workers,
                          int variant);
 /* Launch shapes of the update kernel in this build: threads per CTA and the
@@ -407,7 +408,7 @@ int sbc_read_counters(sbc_forest *f, int64_t *vertices, int64_t *edges, int64_t 
  * stood.  All synchronous. */
 typedef struct sbc_checkpoint sbc_checkpoint;
 int sbc_checkpoint_take(sbc_forest *f, sbc_checkpoint **out);
-/* variant -1: the default update launch shape. */
+/* variant -1: as sbc_forest_create_ex. */
 int sbc_checkpoint_restore(const sbc_checkpoint *c, int variant, sbc_graph **g, sbc_forest **f);
 /* File form: a 40-byte header ("SBCCKPT1", version 1, nv, nk, ne), then off,
  * adj (int32), roots, bc, dist, sigma, delta, little-endian. */

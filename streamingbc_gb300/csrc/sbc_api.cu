@@ -789,7 +789,9 @@ int sbc_forest_create_ex(sbc_forest** out, sbc_graph* g, int64_t nk, const int64
     *out = nullptr;
     if (variant < 0) {
         const char* env = getenv("SBC_UPDATE_VARIANT");
-        variant = env ? atoi(env) : sbc::update_default_variant();
+        int64_t slots = 0;
+        for (int64_t d : g->h_deg_ub) slots += d;
+        variant = env ? atoi(env) : sbc::update_variant_for(slots);
     }
     if (variant < 0 || variant >= sbc::update_variant_count())
         return fail(SBC_ERR_ARG, "update variant %d out of range", variant);

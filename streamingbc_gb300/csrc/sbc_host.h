@@ -381,6 +381,8 @@ inline ForestSlot forest_slot(const sbc_forest* f, int n)
 
 int update_variant_count();
 int update_default_variant();
+// The update shape of a forest created without one, on a graph of that many adjacency slots.
+int update_variant_for(int64_t slots);
 int update_variant_threads(int v);
 int update_workers_per_sm(int v);
 // Sets the calling thread's sbc_last_error() message and returns code.

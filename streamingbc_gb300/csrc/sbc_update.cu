@@ -207,12 +207,30 @@ static const UpdateVariant kVariants[] = {
     {256, 4, 2, launch_variant<256, 4, 2>, occupancy_variant<256, 4, 2>},
 };
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
-// 1024 threads x 1 CTA per SM measured fastest on R-MAT scale 20, K = 1024
-// (531 insertions/s against 413 for 512x2 and 281 for 256x4): with one root in
-// flight per SM, the in-flight one-byte distance rows (152 x 1 MB) about fit
-// the 129 MB L2, so repeated scans of the same hub ancestors within a root's
-// batch hit L2 instead of HBM.
-constexpr int kDefaultVariant = 7;
+constexpr int kDefaultVariant = 7;  // 1024 threads, one root per SM
+
+// The shape of a forest created without one, by the adjacency slots of its
+// graph (what a root's walks can scan).  Measured, insert / delete of a batch in
+// us, 128x8 (2 slots in flight) | 256x4 (2) | 512x2 | 1024x1:
+//   ER 1024 K=1024, 16 k slots         1431/912 | 1606/965 | 2474/1261 | 4075/1948
+//   ER 4000 K=500, 40 k                1238/1008 | 960/1019 | 1230/1081 | 1945/1344
+//   Chung-Lu 5k K=400, 50 k            1079/1079 | 856/1058 | 907/1083 | 1337/1341
+//   R-MAT 13 K=300, 131 k              1017/1192 | 792/1007 | 742/927 | 854/973
+//   Chung-Lu 40k K=256, 352 k          2205/2498 | 1687/1851 | 1623/1709 | 2306/2719
+//   Chung-Lu 100k K=300, 1.2 M         3462/3961 | 2249/2384 | 1958/2080 | 2400/2980
+//   R-MAT 16 K=300, 2 M                2202/2767 | 1488/1533 | 1056/1196 | 1027/1486
+//   R-MAT 17 K=301, 4 M                4035/4439 | 2350/2630 | 1571/1742 | 1332/1752
+//   R-MAT 19 K=300, 16 M               18587/25045 | 10589/11998 | 6358/7294 | 5067/5179
+// Small graphs are bound by the latency of a job's steps, so more roots in
+// flight; from about 1.5 M slots on the walks of a job are, so the whole SM on
+// one root (and its gathered rows stay in L2).
+int update_variant_for(int64_t slots)
+{
+    if (slots < 24000) return 12;      // 128 x 8
+    if (slots < 100000) return 13;     // 256 x 4
+    if (slots < 1500000) return 5;     // 512 x 2
+    return kDefaultVariant;
+}
 
 // Deletion of (u, v), already removed from the adjacency: warp per root.  A
 // root whose endpoints sit on the same level (or are both unreachable) is
