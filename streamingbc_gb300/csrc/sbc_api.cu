@@ -84,7 +84,7 @@ int ensure_staging(sbc_graph* g, int64_t n)
     g->d_ins = nullptr;
     g->h_ins = nullptr;
     CK(dev_alloc(&g->d_ins, (size_t)5 * cap + 1));  // u, v, codes, two rank rows and a flag (launch_append)
-    CK(cudaMallocHost((void**)&g->h_ins, sizeof(int32_t) * 3 * (size_t)cap));
+    CK(cudaMallocHost((void**)&g->h_ins, sizeof(int32_t) * (4 * (size_t)cap + kCallResultInts)));
     g->ins_capacity = cap;
     return SBC_OK;
 }
@@ -180,39 +180,71 @@ int stage_host(sbc_graph* g, int64_t n, const int64_t* u, const int64_t* v, bool
             hv[i] = -1;
         }
     }
-    CK(cudaMemcpyAsync(g->d_ins, hu, sizeof(int32_t) * n, cudaMemcpyHostToDevice, g->stream));
-    CK(cudaMemcpyAsync(g->d_ins + cap, hv, sizeof(int32_t) * n, cudaMemcpyHostToDevice, g->stream));
-    if (set_ok) CK(cudaMemcpyAsync(g->d_ins + 2 * cap, hok, sizeof(int32_t) * n, cudaMemcpyHostToDevice, g->stream));
+    // the rows in one copy
+    const size_t pitch = sizeof(int32_t) * (size_t)cap;
+    CK(cudaMemcpy2DAsync(g->d_ins, pitch, hu, pitch, sizeof(int32_t) * (size_t)n, set_ok ? 3 : 2, cudaMemcpyHostToDevice,
+                         g->stream));
     CK(cudaEventRecord(g->staged, g->stream));
     return SBC_OK;
 }
 
-int collect_stats(sbc_forest* f, int64_t n, sbc_batch_stats* st)
+// Queues the copies of a call's codes (in the staging's third row) and counters
+// into the graph's pinned result block; the counters start again from zero.
+int queue_results(sbc_forest* f, int64_t n, bool counters)
 {
     sbc_graph* g = f->g;
-    if (!st) return SBC_OK;
-    std::vector<int32_t> ok(n);
-    if (n) CK(cudaMemcpyAsync(ok.data(), g->d_ins + 2 * g->ins_capacity, sizeof(int32_t) * n, cudaMemcpyDeviceToHost,
-                              g->stream));
-    int nwork = 0;
-    CK(cudaMemcpyAsync(&nwork, f->d_nwork, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
-    unsigned long long c[SBC_NCOUNTERS];
-    CK(cudaMemcpyAsync(c, f->d_counters, sizeof c, cudaMemcpyDeviceToHost, g->stream));
-    CK(cudaMemsetAsync(f->d_counters, 0, sizeof c, g->stream));
-    CK(cudaStreamSynchronize(g->stream));
+    CallResult* R = g->h_result();
+    CK(cudaMemcpyAsync(g->h_codes(), g->d_ins + 2 * g->ins_capacity, sizeof(int32_t) * n, cudaMemcpyDeviceToHost,
+                       g->stream));
+    if (counters) {
+        CK(cudaMemcpyAsync(R->counters, f->d_counters, sizeof R->counters, cudaMemcpyDeviceToHost, g->stream));
+        CK(cudaMemsetAsync(f->d_counters, 0, sizeof R->counters, g->stream));
+    }
+    return SBC_OK;
+}
+
+void fill_stats(const sbc_graph* g, int64_t n, const unsigned long long* c, sbc_batch_stats* st)
+{
     memset(st, 0, sizeof *st);
+    const int32_t* codes = g->h_codes();
     for (int64_t i = 0; i < n; ++i) {
-        if (ok[i] > 0) st->inserted++;
-        else if (ok[i] == 0) st->duplicates++;
+        if (codes[i] > 0) st->inserted++;
+        else if (codes[i] == 0) st->duplicates++;
         else st->invalid++;
     }
-    st->roots_active = nwork;
     st->vertices = (int64_t)c[0];
     st->edges = (int64_t)c[1];
     st->case1 = (int64_t)c[2];
     st->case2 = (int64_t)c[3];
     st->scanned = (int64_t)c[4];
-    return SBC_OK;
+}
+
+int graph_err(sbc_graph* g, int err)
+{
+    if (!err) return SBC_OK;
+    cudaMemsetAsync(g->d_err, 0, sizeof(int), g->stream);
+    return fail(SBC_ERR_STATE, "adjacency slack exhausted during an insertion batch (reserve capacity first)");
+}
+
+// Waits for an insertion batch: its statistics (st may be null) and, with
+// `check`, the graph's error flag, in one wait.
+int finish_insert(sbc_forest* f, int64_t n, sbc_batch_stats* st, bool check)
+{
+    sbc_graph* g = f->g;
+    CallResult* R = g->h_result();
+    if (st) {
+        int rc = queue_results(f, n, true);
+        if (rc) return rc;
+        CK(cudaMemcpyAsync(&R->nwork, f->d_nwork, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+    }
+    R->err = 0;
+    if (check) CK(cudaMemcpyAsync(&R->err, g->d_err, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+    CK(cudaStreamSynchronize(g->stream));
+    if (st) {
+        fill_stats(g, n, R->counters, st);
+        st->roots_active = R->nwork;
+    }
+    return graph_err(g, R->err);
 }
 
 // One device-input batch: the endpoints' addresses are recorded on the stream
@@ -273,14 +305,10 @@ int replay_batch(sbc_forest* f, int n, const int32_t* d_u, const int32_t* d_v)
 
 int check_graph_err(sbc_graph* g)
 {
-    int err = 0;
-    CK(cudaMemcpyAsync(&err, g->d_err, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+    CallResult* R = g->h_result();
+    CK(cudaMemcpyAsync(&R->err, g->d_err, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
     CK(cudaStreamSynchronize(g->stream));
-    if (err) {
-        cudaMemsetAsync(g->d_err, 0, sizeof(int), g->stream);
-        return fail(SBC_ERR_STATE, "adjacency slack exhausted during an insertion batch (reserve capacity first)");
-    }
-    return SBC_OK;
+    return graph_err(g, R->err);
 }
 
 void free_scratch(sbc_forest* f)
@@ -965,8 +993,7 @@ int sbc_insert_batch(sbc_forest* f, int64_t n, const int64_t* u, const int64_t* 
     CK(sbc::launch_update(f, (int)n, false));
     CK(sbc::launch_seal(g, (int)n));
     f->prof_end(sbc::PROF_BATCH);
-    if ((rc = collect_stats(f, n, stats))) return rc;
-    return check_graph_err(g);
+    return finish_insert(f, n, stats, true);
 }
 
 int sbc_insert_batch_async(sbc_forest* f, int64_t n, const int64_t* u, const int64_t* v)
@@ -1184,36 +1211,12 @@ int sbc_graph_remove_directed(sbc_graph* g, int64_t from, int64_t to, int* resul
     CK(sbc::launch_remove(g, (int)from, (int)to, true, g->d_err + 1));
     CK(cudaMemcpyAsync(result, g->d_err + 1, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
     CK(cudaStreamSynchronize(g->stream));
-    if (*result == 1) g->edge_skew -= sbc::edge_mix((int)from, (int)to);
-    return SBC_OK;
-}
-
-namespace {
-// Deletion statistics of one call from the per-deletion removal codes
-// (staged at d_codes) and the forest's counters.
-int deletion_stats(sbc_forest* f, int64_t n, const int32_t* d_codes, sbc_batch_stats* st)
-{
-    sbc_graph* g = f->g;
-    std::vector<int32_t> codes(n);
-    unsigned long long c[SBC_NCOUNTERS];
-    CK(cudaMemcpyAsync(codes.data(), d_codes, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, g->stream));
-    CK(cudaMemcpyAsync(c, f->d_counters, sizeof c, cudaMemcpyDeviceToHost, g->stream));
-    CK(cudaMemsetAsync(f->d_counters, 0, sizeof c, g->stream));
-    CK(cudaStreamSynchronize(g->stream));
-    memset(st, 0, sizeof *st);
-    for (int32_t k : codes) {
-        if (k > 0) st->inserted++;
-        else if (k == 0) st->duplicates++;
-        else st->invalid++;
+    if (*result == 1) {
+        g->edge_skew -= sbc::edge_mix((int)from, (int)to);
+        g->h_deg_ub[from]--;
     }
-    st->vertices = (int64_t)c[0];
-    st->edges = (int64_t)c[1];
-    st->case1 = (int64_t)c[2];
-    st->case2 = (int64_t)c[3];
-    st->scanned = (int64_t)c[4];
     return SBC_OK;
 }
-}  // namespace
 
 int sbc_delete_batch(sbc_forest* f, int64_t n, const int64_t* u, const int64_t* v, sbc_batch_stats* stats)
 {
@@ -1229,7 +1232,7 @@ int sbc_delete_batch(sbc_forest* f, int64_t n, const int64_t* u, const int64_t* 
     }
     int rc = stage_host(g, n, u, v, false);
     if (rc) return rc;
-    const int32_t* codes = g->d_ins + 2 * g->ins_capacity;
+    CallResult* R = g->h_result();
     if (stats) CK(cudaMemsetAsync(f->d_counters, 0, sizeof(unsigned long long) * SBC_NCOUNTERS, g->stream));
     // the whole batch in one update launch: removals marked in order, every
     // root through the deletions in order (each job seeing the graph as it
@@ -1238,9 +1241,33 @@ int sbc_delete_batch(sbc_forest* f, int64_t n, const int64_t* u, const int64_t* 
     CK(sbc::launch_mark_removed(g, (int)n));
     CK(sbc::launch_delete_batch(f, (int)n));
     CK(sbc::launch_compact_removed(g, (int)n));
-    CK(sbc::launch_delete_finish(f));
-    if (stats) return deletion_stats(f, n, codes, stats);
+    if ((rc = queue_results(f, n, stats != nullptr))) return rc;
+    CK(cudaMemcpyAsync(&R->dirty, f->d_dcnt, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
     CK(cudaStreamSynchronize(g->stream));
+    // the host's degree bounds follow the removals (without that a window of
+    // edges that come and go re-packed the adjacency every few steps)
+    const int32_t* codes = g->h_codes();
+    for (int64_t i = 0; i < n; ++i)
+        if (codes[i] > 0) {
+            g->h_deg_ub[u[i]]--;
+            g->h_deg_ub[v[i]]--;
+        }
+    if (stats) fill_stats(g, n, R->counters, stats);
+    if (R->dirty > 0) {
+        CK(sbc::launch_delete_finish(f, R->dirty));
+        if (stats) {  // the recomputes count as traversals
+            CK(cudaMemcpyAsync(R->counters, f->d_counters, sizeof R->counters, cudaMemcpyDeviceToHost, g->stream));
+            CK(cudaMemsetAsync(f->d_counters, 0, sizeof R->counters, g->stream));
+        }
+        CK(cudaStreamSynchronize(g->stream));
+        if (stats) {
+            stats->vertices += (int64_t)R->counters[0];
+            stats->edges += (int64_t)R->counters[1];
+            stats->case1 += (int64_t)R->counters[2];
+            stats->case2 += (int64_t)R->counters[3];
+            stats->scanned += (int64_t)R->counters[4];
+        }
+    }
     return SBC_OK;
 }
 
@@ -1256,8 +1283,16 @@ int sbc_update_deleted(sbc_forest* f, int64_t u, int64_t v, sbc_batch_stats* sta
     CK(cudaMemcpyAsync(g->d_err + 1, &kRemoved, sizeof(int), cudaMemcpyHostToDevice, g->stream));
     if (stats) CK(cudaMemsetAsync(f->d_counters, 0, sizeof(unsigned long long) * SBC_NCOUNTERS, g->stream));
     CK(sbc::launch_delete(f, (int)u, (int)v, g->d_err + 1));
-    if (stats) return deletion_stats(f, 1, g->d_err + 1, stats);
+    CallResult* R = g->h_result();
+    if (stats) {
+        CK(cudaMemcpyAsync(R->counters, f->d_counters, sizeof R->counters, cudaMemcpyDeviceToHost, g->stream));
+        CK(cudaMemsetAsync(f->d_counters, 0, sizeof R->counters, g->stream));
+    }
     CK(cudaStreamSynchronize(g->stream));
+    if (stats) {
+        g->h_codes()[0] = 1;
+        fill_stats(g, 1, R->counters, stats);
+    }
     return SBC_OK;
 }
 
@@ -1863,9 +1898,7 @@ int sbc_update_inserted(sbc_forest* f, int64_t n, const int64_t* u, const int64_
     f->prof_begin(sbc::PROF_BATCH);
     CK(sbc::launch_update(f, (int)n, true));
     f->prof_end(sbc::PROF_BATCH);
-    if (stats) return collect_stats(f, n, stats);
-    CK(cudaStreamSynchronize(g->stream));
-    return SBC_OK;
+    return finish_insert(f, n, stats, false);
 }
 
 int sbc_sync(sbc_forest* f)

@@ -117,6 +117,14 @@ struct WorkerScratch {
     }
 };
 
+// What a synchronous call reads back beside its codes, into pinned memory, so
+// that one wait serves all of it (a copy to pageable memory waits by itself).
+struct CallResult {
+    unsigned long long counters[SBC_NCOUNTERS];
+    int nwork, err, dirty;
+};
+constexpr size_t kCallResultInts = (sizeof(CallResult) + 3) / 4;
+
 // Device-resident slack-CSR adjacency (replaces the STINGER edge-block store,
 // src/stinger/stinger-internal.h:45-103).  All device work for the graph and
 // for forests bound to it runs on `stream`, in order.
@@ -140,7 +148,7 @@ struct sbc_graph {
     // staging for insertion batches
     int ins_capacity = 0;
     int32_t* d_ins = nullptr;  // [5 * ins_capacity + 1]: u, v, ok, then the append's ranks and misfit flag
-    int32_t* h_ins = nullptr;  // pinned [3 * ins_capacity]
+    int32_t* h_ins = nullptr;  // pinned: staging [3 * ins_capacity], a call's codes [ins_capacity], its CallResult
     cudaEvent_t staged = nullptr;  // recorded after the last copy out of h_ins
     const int32_t** d_src = nullptr;  // device slot: addresses of the caller's endpoint arrays
     int64_t repacks = 0;
@@ -149,6 +157,8 @@ struct sbc_graph {
     bool last_directed = false;  // the staged insertions were appended one direction only
     unsigned long long edge_skew = 0;  // edge_mix summed over the live slots: 0 when every edge has both directions
 
+    int32_t* h_codes() const { return h_ins + 3 * (size_t)ins_capacity; }
+    CallResult* h_result() const { return reinterpret_cast<CallResult*>(h_ins + 4 * (size_t)ins_capacity); }
     sbc::DevGraph dev() const
     {
         sbc::DevGraph G;
@@ -412,10 +422,10 @@ cudaError_t launch_remove(sbc_graph* g, int u, int v, bool directed, int* d_res)
 // down or are recomputed from scratch (SBC_DELETE_*), a recomputed root's old
 // dependencies taken out of BC first.
 // launch_delete_step: the update of one deletion, recomputes left for
-// launch_delete_finish, which recomputes the listed roots once on the graph as
+// launch_delete_finish, which recomputes the n listed roots once on the graph as
 // it then stands and puts their rows back.
 cudaError_t launch_delete_step(sbc_forest* f, int u, int v, const int* d_removed);
-cudaError_t launch_delete_finish(sbc_forest* f);
+cudaError_t launch_delete_finish(sbc_forest* f, int n);
 cudaError_t launch_delete(sbc_forest* f, int u, int v, const int* d_removed);
 // Every root through the n deletions marked in g's staging (launch_mark_removed),
 // in one persistent launch; dirty roots are left for launch_delete_finish.

@@ -388,14 +388,11 @@ cudaError_t launch_delete_step(sbc_forest* f, int u, int v, const int* d_removed
     return cudaGetLastError();
 }
 
-cudaError_t launch_delete_finish(sbc_forest* f)
+cudaError_t launch_delete_finish(sbc_forest* f, int n)
 {
     sbc_graph* g = f->g;
     cudaStream_t s = g->stream;
     cudaError_t e;
-    int n = 0;
-    if ((e = cudaMemcpyAsync(&n, f->d_dcnt, sizeof(int), cudaMemcpyDeviceToHost, s)) || (e = cudaStreamSynchronize(s)))
-        return e;
     if (n == 0) return cudaSuccess;
     // a few roots of a large graph: one at a time by the whole GPU (a CTA
     // would walk the whole graph alone); otherwise a CTA per root
@@ -484,7 +481,11 @@ cudaError_t launch_delete(sbc_forest* f, int u, int v, const int* d_removed)
 {
     cudaError_t e = launch_delete_step(f, u, v, d_removed);
     if (e) return e;
-    return launch_delete_finish(f);
+    int n = 0;
+    if ((e = cudaMemcpyAsync(&n, f->d_dcnt, sizeof(int), cudaMemcpyDeviceToHost, f->g->stream)) ||
+        (e = cudaStreamSynchronize(f->g->stream)))
+        return e;
+    return launch_delete_finish(f, n);
 }
 
 }  // namespace sbc
