@@ -403,9 +403,9 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
                 const int64_t rrow = A.G.row[root];
                 const int rdeg = vis_deg(A.G, root, rrow, g);
                 const bool rootDown = (W.st[root] & SBC_STEP_MASK) != 0;
-                // the loop below claims (masks) or lists vertices: every thread
-                // has read the counts of the level before
-                if (L == 2) __syncthreads();
+                // what follows claims vertices without another barrier: every
+                // thread has read the count of the level before
+                __syncthreads();
                 long long push_cost = 0, mixed_cost = 0;
                 double root_sum = 0.0;
                 const int qbase = sm.st;  // free tail of the same-level queue holds the two lists
