@@ -161,10 +161,8 @@ struct ScratchBase {
 // appended in sequence order, so those are a prefix of [deg0, deg): found by
 // binary search (a hub can take dozens of a batch's insertions; one dependent
 // load per appended slot was a long serial chain on every visit).
-__device__ __forceinline__ int vis_deg(const DevGraph& G, int x, int64_t rs, int g)
+__device__ __forceinline__ int vis_deg_of(const DevGraph& G, int64_t rs, int d0, int d, int g)
 {
-    const int d0 = G.deg0[x];
-    const int d = G.deg[x];
     if (d0 == d || g == INT_MAX) return d;
     int lo = d0, hi = d;  // first slot in [d0, d) with seq > g
     while (lo < hi) {
@@ -173,6 +171,11 @@ __device__ __forceinline__ int vis_deg(const DevGraph& G, int x, int64_t rs, int
         else hi = mid;
     }
     return lo;
+}
+
+__device__ __forceinline__ int vis_deg(const DevGraph& G, int x, int64_t rs, int g)
+{
+    return vis_deg_of(G, rs, G.deg0[x], G.deg[x], g);
 }
 
 // Is y among the first vx (visible) neighbours of x, whose slots start at rx?
@@ -449,6 +452,61 @@ __device__ __forceinline__ void lb_walk(const DevGraph& G, int g, const DistRow 
 struct NoPost {
     __device__ void operator()(int, int) const {}
 };
+
+// lb_walk for the short levels that most of a job's steps are: their time is one
+// chain of dependent loads after the other, so what does not depend on a chain
+// is loaded beside it.  load(x) is called as soon as x is known, next to the
+// loads of its degree, and its value handed to prep(j, x, degree, value); and
+// where the chunk has at most one slot per thread, aux(k) is loaded with the
+// neighbour's distance and handed to edge(j, x, k, dist[k], aux), which gets
+// kNoAux for longer chunks (there most neighbours fail the distance test, and
+// edge loads it itself).  Values that may change meanwhile are edge's to check.
+constexpr int kNoAux = -1;
+template <int NT, int ILP, bool TOMB, class Load, class Prep, class Aux, class Edge>
+__device__ __forceinline__ void lb_walk_ahead(const DevGraph& G, int g, const DistRow dr, const int32_t* l1, int n1,
+                                              const int32_t* l2, int n2, LbSmem<NT>& sm, Load load, Prep prep, Aux aux,
+                                              Edge edge)
+{
+    const int n = n1 + n2;
+    for (int base = 0; base < n; base += NT) {
+        const int t = threadIdx.x;
+        const int cnt = min(NT, n - base);
+        int d = 0;
+        if (t < cnt) {
+            const int idx = base + t;
+            const int x = idx < n1 ? l1[idx] : l2[idx - n1];
+            const int64_t rs = G.row[x];
+            const int d0 = G.deg0[x], dx = G.deg[x];
+            auto value = load(x);
+            d = vis_deg_of(G, rs, d0, dx, g);
+            sm.x[t] = x;
+            sm.row[t] = rs;
+            prep(t, x, d, value);
+        }
+        int total;
+        const int off = block_exclusive_scan<NT>(d, sm.warp, &total);
+        if (t < cnt) sm.off[t] = off;
+        if (t == 0) {
+            sm.off[cnt] = total;
+            sm.walked_v += (unsigned)cnt;
+            sm.walked_e += (unsigned)total;
+            sm.scanned_e += (unsigned)total;
+        }
+        __syncthreads();
+        int j = 0;  // chunk vertex of this thread's current edge; edges only move forward
+        const int per = min(ILP, (total + NT - 1) / NT);
+        for (int e0 = t * per; e0 < total; e0 += NT * per) {
+            int kk[ILP], jj[ILP], dk[ILP];
+            walk_fetch<NT, ILP, TOMB>(G, sm, cnt, total, e0, per, g, j, kk, jj);
+            const int a = per == 1 && kk[0] >= 0 ? aux(kk[0]) : kNoAux;
+            gather_dist<ILP>(dr, kk, dk);
+#pragma unroll
+            for (int u = 0; u < ILP; ++u)
+                if (kk[u] >= 0) edge(jj[u], sm.x[jj[u]], kk[u], dk[u], u == 0 ? a : kNoAux);
+        }
+        __syncthreads();
+    }
+}
 
 // Edge-balanced walk that sums one value per edge into the edge's source
 // vertex: contrib(j, y, k, dist[k], v) returns whether edge (y,k) contributes

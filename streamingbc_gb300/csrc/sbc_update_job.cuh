@@ -27,6 +27,14 @@ struct UpdSmem {
 // many times the root's degree; a probe is costed as this many scanned slots.
 constexpr int kProbeRatio = 32;
 
+// What a commit reads of a vertex.
+struct Committed {
+    int st;
+    int64_t sigma;
+    double delta, acc;
+    int64_t dp;
+};
+
 template <int NT, int ILP, bool DECR, bool TOMB>
 __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, const Scratch& W, int r, int a, int b,
                                        bool moving, int g, bool del, int Lb, int nsteps, int ndown);
@@ -69,12 +77,13 @@ __device__ __forceinline__ void run_job(const ForestSlot& A, UpdSmem<NT>& sm, co
         const int L = Lb + step;
         const int tag = step + 2;
         // a re-levelling descent compares old distances far from L: one-byte row
-        lb_walk<NT, true, ILP, TOMB>(
+        lb_walk_ahead<NT, ILP, TOMB>(
             A.G, g, DistRow{D, D8, moving ? nullptr : D2, L}, W.qd + lo, hi - lo, nullptr, 0, sm.lb,
-            [&](int j, int x, int d) { sm.dp[j] = W.dp[x]; },
-            [&](int j, int x, int k, int dk) {
+            [&](int x) { return W.dp[x]; }, [&](int j, int x, int d, int64_t dp) { sm.dp[j] = dp; },
+            [&](int k) { return W.st[k]; },
+            [&](int j, int x, int k, int dk, int sk) {
                 if (moving ? (dk <= L) : (dk != L + 1)) return;
-                int s = W.st[k];
+                int s = sk != kNoAux ? sk : W.st[k];
                 if (s == 0) {
                     const int old = atomicCAS(&W.st[k], 0, tag);
                     warp_append(&sm.qt, W.qd, k, old == 0);
@@ -82,8 +91,7 @@ __device__ __forceinline__ void run_job(const ForestSlot& A, UpdSmem<NT>& sm, co
                 }
                 if ((s & SBC_STEP_MASK) != tag) return;
                 atomic_add_i64(&W.dp[k], sm.dp[j]);
-            },
-            NoPost());
+            });
         lo = hi;
         hi = sm.qt;
         ++step;
@@ -163,14 +171,14 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
     int L = 0;
     // Finalise vertex x of the level being walked: new sigma/delta committed in
     // place, BC += newdelta - olddelta, and its child weights wn, wd returned.
-    auto commit = [&](int x, double& wn, double& wd) {
-        const int s = W.st[x];
+    auto load = [&](int x) { return Committed{W.st[x], S[x], Dl[x], W.acc[x], W.dp[x]}; };
+    auto commit = [&](int x, const Committed& v, double& wn, double& wd) {
+        const int s = v.st;
         const bool isDown = (s & SBC_STEP_MASK) != 0;
         const bool mv = (s & SBC_MOVED) != 0;
-        const int64_t oS = S[x];
-        const double oD = Dl[x];
-        const double ac = W.acc[x];
-        const int64_t nS = isDown ? (mv ? W.dp[x] : oS + W.dp[x]) : oS;
+        const int64_t oS = v.sigma;
+        const double oD = v.delta, ac = v.acc;
+        const int64_t nS = isDown ? (mv ? v.dp : oS + v.dp) : oS;
         const Sigma ws = sigma_of(nS);
         const double nD = isDown ? ws.b * ac : oD + ws.b * ac;
         wn = child_weight(nD + 1.0, ws);
@@ -182,12 +190,12 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
         // is claimed when its level has been walked
         if (!DECR && del && x == b) atomicAdd(&W.acc[a], wd - wn);
     };
-    auto prep = [&](int j, int x, int d) {
+    auto prep = [&](int j, int x, int d, const Committed& v) {
         double wn, wd;
-        commit(x, wn, wd);
+        commit(x, v, wn, wd);
         sm.wn[j] = wn;
         sm.wd[j] = wd;
-        sm.fl[j] = ((W.st[x] & SBC_MOVED) ? 1 : 0) | (x == b ? 2 : 0);
+        sm.fl[j] = ((v.st & SBC_MOVED) ? 1 : 0) | (x == b ? 2 : 0);
     };
     // Child weights of an already committed vertex, kept in its acc/dp slots.
     auto prep_loaded = [&](int j, int x, int d) {
@@ -195,9 +203,10 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
         sm.wd[j] = __longlong_as_double((long long)W.dp[x]);
         sm.fl[j] = ((W.st[x] & SBC_MOVED) ? 1 : 0) | (x == b ? 2 : 0);
     };
-    auto parent_edge = [&](int j, int x, int k, int dk) -> bool {
+    auto state = [&](int k) { return W.st[k]; };
+    auto parent_edge = [&](int j, int x, int k, int dk, int known) -> bool {
         if (dk != L - 1) return false;
-        const int sk = W.st[k];
+        const int sk = known != kNoAux ? known : W.st[k];
         const bool kDown = (sk & SBC_STEP_MASK) != 0;
         if (!kDown && !(sk & SBC_ASC)) {
             const int old = atomicOr(&W.st[k], SBC_ASC);
@@ -290,8 +299,8 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
     // roster.  The reference edge counter still counts its full degree.
     const int32_t* rcand = nullptr;
     int rcnt = 0;
-    auto prep_div = [&](int j, int x, int& d) {
-        prep(j, x, d);
+    auto prep_div = [&](int j, int x, int& d, const Committed& v) {
+        prep(j, x, d, v);
         if (rcand && (long long)d > (long long)kProbeRatio * rcnt) {
             W.acc[x] = sm.wn[j];
             W.dp[x] = (int64_t)__double_as_longlong(sm.wd[j]);
@@ -351,27 +360,26 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
             int nn1 = dn, nn2 = ua_hi - ua_lo;
             bool near = pull_ok;
             if (!pull_ok && (!moving || DECR)) {
-                lb_walk<NT, true, ILP, TOMB>(A.G, g, DistRow{D, D8, D2, L}, dlist, dn, W.qa + ua_lo, ua_hi - ua_lo, sm.lb,
-                                       prep_div,
-                                       [&](int j, int x, int k, int dk) { parent_edge(j, x, k, dk); }, NoPost());
+                lb_walk_ahead<NT, ILP, TOMB>(A.G, g, DistRow{D, D8, D2, L}, dlist, dn, W.qa + ua_lo, ua_hi - ua_lo, sm.lb,
+                                             load, prep_div, state,
+                                             [&](int j, int x, int k, int dk, int sk) { parent_edge(j, x, k, dk, sk); });
                 probe_diverted();
             } else if (!pull_ok) {
                 const int same_lo = sm.st;
-                lb_walk<NT, true, ILP, TOMB>(
-                    A.G, g, DistRow{D, D8, D2, L}, dlist, dn, nullptr, 0, sm.lb, prep,
-                    [&](int j, int x, int k, int dk) {
-                        if (parent_edge(j, x, k, dk)) return;
+                lb_walk_ahead<NT, ILP, TOMB>(
+                    A.G, g, DistRow{D, D8, D2, L}, dlist, dn, nullptr, 0, sm.lb, load, prep, state,
+                    [&](int j, int x, int k, int dk, int known) {
+                        if (parent_edge(j, x, k, dk, known)) return;
                         if (!(sm.fl[j] & 1) || dk != L) return;
                         // k kept its level and lost the moved vertex x as a child
-                        const int sk = W.st[k];
+                        const int sk = known != kNoAux ? known : W.st[k];
                         if (sk & SBC_STEP_MASK) return;
                         if (!(sk & SBC_ASC)) {
                             const int old = atomicOr(&W.st[k], SBC_ASC);
                             warp_append(&sm.st, W.qs, k, !(old & SBC_ASC));
                         }
                         atomicAdd(&W.acc[k], sm.wd[j] - sm.wn[j]);
-                    },
-                    NoPost());
+                    });
                 const int same_hi = sm.st;
                 const int n2w = ua_hi - ua_lo + same_hi - same_lo;
                 // level 2 keeps its scan list after the same-level entries of
@@ -383,9 +391,10 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
                     nl2 = W.qs + same_lo;
                     nn2 = same_hi - same_lo;
                 } else {
-                    lb_walk<NT, true, ILP, TOMB>(A.G, g, DistRow{D, D8, D2, L}, W.qa + ua_lo, ua_hi - ua_lo, W.qs + same_lo,
-                                           same_hi - same_lo, sm.lb, prep_div,
-                                           [&](int j, int x, int k, int dk) { parent_edge(j, x, k, dk); }, NoPost());
+                    lb_walk_ahead<NT, ILP, TOMB>(
+                        A.G, g, DistRow{D, D8, D2, L}, W.qa + ua_lo, ua_hi - ua_lo, W.qs + same_lo, same_hi - same_lo, sm.lb,
+                        load, prep_div, state,
+                        [&](int j, int x, int k, int dk, int sk) { parent_edge(j, x, k, dk, sk); });
                     probe_diverted();
                 }
             }
@@ -416,7 +425,7 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
                     const int xd0 = A.G.deg0[x], xd = A.G.deg[x];
                     const unsigned m0 = (L == 2 && M2) ? M2[x] : 0u;
                     double wn, wd;
-                    commit(x, wn, wd);
+                    commit(x, load(x), wn, wd);
                     W.acc[x] = wn;
                     W.dp[x] = (int64_t)__double_as_longlong(wd);
                     const int dx = (xd0 == xd || g == INT_MAX) ? xd : vis_deg(A.G, x, rx, g);
@@ -505,7 +514,8 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
                         const int nscan = sm.nscan, nprobe = sm.nprobe;
                         lb_walk<NT, false, ILP, TOMB>(A.G, g, DistRow{D, D8, D2, L}, W.qs + qbase, nscan, nullptr, 0, sm.lb,
                                                 prep_loaded,
-                                           [&](int j, int x, int k, int dk) { parent_edge(j, x, k, dk); }, NoPost());
+                                           [&](int j, int x, int k, int dk) { parent_edge(j, x, k, dk, kNoAux); },
+                                                NoPost());
                         probe_parents(W.qs + nv - nprobe, nprobe, A.G.col + rrow, rdeg, TOMB);
                     }
                     for (int i = threadIdx.x; i < nn1 + nn2; i += NT) {
