@@ -1,17 +1,17 @@
 // Static Brandes initialisation over K roots.
 //
 // Replaces BrandesApproxCaseParallel / BrandesSingleTree
-// (src/streamingbc_init.c:60-84, :87-183).  One persistent CTA per worker slot
-// takes roots from an atomic counter.  Per root:
-//   forward   level-synchronous BFS; a frontier vertex pushes its sigma into
-//             every neighbour on the next level (int64 atomics, so the sum is
-//             exact and order-independent); the first visitor of a vertex
-//             claims it with a CAS on dist and appends it to the next frontier.
-//   backward  levels from deepest to 0, pull form: a vertex x sums
-//             w[c] = (delta[c]+1)/sigma[c] over its children c (dist[c] =
-//             dist[x]+1) and sets delta[x] = sigma[x] * sum; no global atomics.
+// (src/streamingbc_init.c:60-84, :87-183).  Persistent CTAs take roots from an
+// atomic counter.  Per root (k_static):
+//   forward   level-synchronous BFS; per level the frontier pushes its sigma into
+//             the unvisited neighbours (int64 atomics, exact and
+//             order-independent), or the unvisited vertices pull it, whichever
+//             scans fewer slots.
+//   backward  levels from deepest to 0: delta[x] = sigma[x] * sum over children c
+//             of w[c] = (delta[c]+1)/sigma[c], the sum pulled by the parents or
+//             pushed by the children, again by slots.
 // BC is then a column sum of delta over roots excluding each root itself
-// (init.c:175-177), computed by k_bc_colsum in root order.
+// (init.c:175-177), k_bc_colsum.
 #include <climits>
 #include <mutex>
 #include <string>
@@ -1054,6 +1054,11 @@ StaticShape static_shape(int64_t nv, int64_t nk, int64_t workers, int sm_count, 
     // fewer CTAs while the SM's shared memory does not hold them (1 KB each is the system's)
     while (c > 1 && (size_t)c * (S.dyn + static_fixed(pow2_floor(1024 / c), S.mode) + 1024) > smem_sm) --c;
     S.nt = std::max(pow2_floor(1024 / c), S.mode == kSmall ? 128 : S.mode == kBits ? 256 : 1024);
+    // A small graph's levels are too short for 1,024 threads (barriers and
+    // claims cost more than the extra threads walk): with one CTA per SM,
+    // R-MAT 10, 60 roots 100 us with 256 threads, 126 with 1,024; R-MAT 12
+    // 187 with 512, 199 with 256, 249 with 1,024.
+    if (S.mode == kSmall) S.nt = std::min(S.nt, nv < 2048 ? 256 : 512);
     S.grid = (int)std::min<int64_t>(nk, c * sm_count);
     if (S.mode != kSmall) S.grid = (int)std::min<int64_t>(S.grid, workers * S.halves);
     S.kernel = static_kernel(S.nt, S.mode);
