@@ -68,6 +68,35 @@ __global__ void k_append(int64_t nv, const int64_t* __restrict__ row, int32_t* d
     append_warp(nv, row, deg, cap, col, seq, n, iu, iv, ok, directed, err);
 }
 
+// First slot of x in [0, ns) whose neighbour is >= y, 32 probes a step.
+__device__ __forceinline__ int warp_lower_bound(const int32_t* __restrict__ col, int64_t rx, int ns, int y)
+{
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int lo = 0, hi = ns;
+    while (hi > lo) {
+        const int step = (hi - lo + 31) >> 5;
+        const int64_t p = lo + (int64_t)lane * step;
+        const int below = __popc(__ballot_sync(full, p < hi && col[rx + p] < y));  // probes ascend: the first `below`
+        const int base = lo;
+        if (below == 0) return base;
+        lo = (int)min((int64_t)hi, base + (int64_t)(below - 1) * step + 1);
+        hi = (int)min((int64_t)hi, base + (int64_t)below * step);
+    }
+    return lo;
+}
+
+// Whether y is among x's d slots, the first ns of which are sorted (one warp).
+__device__ __forceinline__ bool has_slot(const int32_t* col, int64_t rx, int ns, int d, int y)
+{
+    const int lane = threadIdx.x & 31;
+    const int p = warp_lower_bound(col, rx, ns, y);
+    bool found = p < ns && col[rx + p] == y;
+    for (int s = ns + lane; s < d; s += 32)
+        if (col[rx + s] == y) found = true;
+    return __any_sync(0xffffffffu, found);
+}
+
 // The same results with a warp per insertion, in three launches:
 //   k_append_codes  -1 bad id or loop; 0 an edge already (of the graph as the
 //                   batch begins -- sealed, so a binary search of the sorted
@@ -114,23 +143,7 @@ __global__ void k_append_codes(int64_t nv, const int64_t* __restrict__ row, cons
         }
         const int64_t rx = row[x];
         const int d = deg[x], ns = min(nsort[x], d);
-        bool found = false;
-        if (lane == 0) {
-            int lo = 0, hi = ns;
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                const int c = col[rx + mid];
-                if (c < y) lo = mid + 1;
-                else if (c > y) hi = mid;
-                else {
-                    found = true;
-                    break;
-                }
-            }
-        }
-        for (int s = ns + lane; s < d; s += 32)
-            if (col[rx + s] == y) found = true;
-        if (__any_sync(0xffffffffu, found)) code = 0;
+        if (has_slot(col, rx, ns, d, y)) code = 0;
     }
     if (lane == 0) ok[w] = code;
 }
@@ -185,12 +198,109 @@ __global__ void k_append_place(int64_t nv, const int64_t* __restrict__ row, int3
     }
 }
 
-// Many graphs' batches at once: one warp (CTA) per graph, each appending its
-// graph's insertions in order exactly as k_append does.
-__global__ void k_append_group(const __grid_constant__ GraphBatchSlots S)
+// The three steps in one CTA, a warp per insertion at a time: the batch and its
+// codes are held in shared memory and barriers stand where the launches were.
+// The time is that of a few dependent loads per round of warps, so a short
+// batch costs one launch instead of three and a graph of a group does not take
+// its insertions one after the other.  With the seal done by the merge: a step
+// of one insertion and one deletion on ER 200 360 -> 347 us; 16 R-MAT graphs,
+// 16 insertions each, where one warp per graph appended for 51 us: 10.28 ->
+// 10.20 ms.  At two rounds of the CTA's 32 warps it measures the same as the
+// three launches (a step of 37 on R-MAT 17 4.67 and 4.66 ms, of 64 on Chung-Lu
+// 40k 4.15 both ways); beyond that a graph's batch keeps the launches.
+constexpr int kBlockAppendMax = 256;  // insertions per CTA
+constexpr int kFusedAppendMax = 64;   // one graph's batch
+
+__device__ __forceinline__ void append_block(int64_t nv, const int64_t* row, int32_t* deg, const int32_t* deg0,
+                                             const int32_t* nsort, const int32_t* cap, int32_t* col, int32_t* seq,
+                                             int n, const int32_t* iu, const int32_t* iv, int32_t* ok, int directed,
+                                             int* err)
+{
+    __shared__ int s_u[kBlockAppendMax], s_v[kBlockAppendMax], s_ok[kBlockAppendMax];
+    __shared__ int s_ru[kBlockAppendMax], s_rv[kBlockAppendMax];
+    __shared__ int s_misfit;
+    const int lane = threadIdx.x & 31, warps = (int)(blockDim.x >> 5);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        s_u[i] = iu[i];
+        s_v[i] = iv[i];
+    }
+    if (threadIdx.x == 0) s_misfit = 0;
+    __syncthreads();
+    for (int w = (int)(threadIdx.x >> 5); w < n; w += warps) {
+        const int u = s_u[w], v = s_v[w];
+        int code = (u == v || u < 0 || v < 0 || u >= nv || v >= nv) ? -1 : 1;
+        if (code == 1) {
+            bool same = false;
+            for (int j = lane; j < w; j += 32)
+                same |= (s_u[j] == u && s_v[j] == v) || (!directed && s_u[j] == v && s_v[j] == u);
+            if (__any_sync(0xffffffffu, same)) code = 0;
+        }
+        if (code == 1) {
+            const bool swap = !directed && deg[v] < deg[u];
+            const int x = swap ? v : u;
+            const int d = deg[x];
+            if (has_slot(col, row[x], min(nsort[x], d), d, swap ? u : v)) code = 0;
+        }
+        if (lane == 0) s_ok[w] = code;
+    }
+    __syncthreads();
+    for (int w = (int)(threadIdx.x >> 5); w < n; w += warps) {
+        if (s_ok[w] != 1) continue;
+        const int u = s_u[w], v = s_v[w];
+        int ru = 0, rv = 0;
+        for (int j = lane; j < w; j += 32) {
+            if (s_ok[j] != 1) continue;
+            ru += (s_u[j] == u || (!directed && s_v[j] == u)) ? 1 : 0;
+            rv += ((!directed && s_u[j] == v) || s_v[j] == v) ? 1 : 0;
+        }
+        ru = __reduce_add_sync(0xffffffffu, ru);
+        rv = __reduce_add_sync(0xffffffffu, rv);
+        if (lane == 0) {
+            s_ru[w] = ru;
+            s_rv[w] = rv;
+            if (deg0[u] + ru >= cap[u] || (!directed && deg0[v] + rv >= cap[v])) s_misfit = 1;
+        }
+    }
+    __syncthreads();
+    if (s_misfit) {
+        // a slot does not fit: the whole batch in order, one warp
+        if (threadIdx.x < 32) append_warp(nv, row, deg, cap, col, seq, n, iu, iv, ok, directed, err);
+        return;
+    }
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        ok[i] = s_ok[i];
+        if (s_ok[i] != 1) continue;
+        const int u = s_u[i], v = s_v[i];
+        const int pu = deg0[u] + s_ru[i];
+        col[row[u] + pu] = v;
+        seq[row[u] + pu] = i;
+        atomicMax(&deg[u], pu + 1);
+        if (!directed) {
+            const int pv = deg0[v] + s_rv[i];
+            col[row[v] + pv] = u;
+            seq[row[v] + pv] = i;
+            atomicMax(&deg[v], pv + 1);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(1024) k_append_small(int64_t nv, const int64_t* row, int32_t* deg,
+                                                       const int32_t* deg0, const int32_t* nsort, const int32_t* cap,
+                                                       int32_t* col, int32_t* seq, int n, const int32_t* iu,
+                                                       const int32_t* iv, int32_t* ok, int directed, int* err)
+{
+    append_block(nv, row, deg, deg0, nsort, cap, col, seq, n, iu, iv, ok, directed, err);
+}
+
+// Many graphs' batches at once, a CTA per graph; a batch too long for the
+// CTA's tables is appended in order by one warp.
+__global__ void __launch_bounds__(1024) k_append_group(const __grid_constant__ GraphBatchSlots S)
 {
     const GraphBatchSlot& b = S.slot[blockIdx.x];
-    append_warp(b.nv, b.row, b.deg, b.cap, b.col, b.seq, b.n, b.iu, b.iv, b.ok, 0, b.err);
+    if (b.n <= kBlockAppendMax)
+        append_block(b.nv, b.row, b.deg, b.deg0, b.nsort, b.cap, b.col, b.seq, b.n, b.iu, b.iv, b.ok, 0, b.err);
+    else if (threadIdx.x < 32)
+        append_warp(b.nv, b.row, b.deg, b.cap, b.col, b.seq, b.n, b.iu, b.iv, b.ok, 0, b.err);
 }
 
 // A batch's endpoint arrays live in the caller's device memory.  k_set_src
@@ -234,8 +344,10 @@ cudaError_t launch_stage(sbc_graph* g, int n)
 // prefix, then a scan of the tail) never scan more than the current batch's
 // appends -- without this a hub's tail grew by every insertion on it.  One
 // block per endpoint of an applied insertion; the first block to reach a
-// vertex claims it by swapping its deg0 for -1 (the seal that follows rewrites
-// deg0 = deg for the same endpoints; the update that read deg0 has finished).
+// vertex claims it by swapping its deg0 for -1 and, when it is done, seals it:
+// deg0 = deg makes the appended slots visible to all later traversals (the
+// update that read deg0 has finished).  A block that finds deg0 = deg comes
+// after the claimer (an appended slot leaves deg0 < deg) and puts it back.
 // The tail (at most kMergeTail slots per batch; a longer one is merged over
 // several batches) is sorted in shared memory; each tail value's final slot is
 // its rank among the tail plus its lower bound in the prefix; prefix values
@@ -253,12 +365,16 @@ __device__ __forceinline__ void merge_tail(const int64_t* __restrict__ row, cons
     __shared__ int s_dst[kMergeTail];
     __shared__ int s_claim;
     const int tid = threadIdx.x;
+    const int dx = deg[x];
     if (tid == 0) s_claim = atomicExch(&deg0[x], -1);
     __syncthreads();
     if (s_claim < 0) return;  // another block merges x
     const int ns = nsort[x];
-    const int t = min(deg[x] - ns, kMergeTail);
-    if (t <= 0) return;
+    const int t = s_claim == dx ? 0 : min(dx - ns, kMergeTail);
+    if (t <= 0) {  // no appended slots, or another block has merged them and left
+        if (tid == 0) deg0[x] = dx;
+        return;
+    }
     const int64_t rx = row[x];
     int P = 1;
     while (P < t) P <<= 1;
@@ -317,7 +433,10 @@ __device__ __forceinline__ void merge_tail(const int64_t* __restrict__ row, cons
         __syncthreads();
     }
     for (int k = tid; k < t; k += kMergeThreads) col[rx + s_dst[k]] = s_tail[k];
-    if (tid == 0) nsort[x] = ns + t;
+    if (tid == 0) {
+        nsort[x] = ns + t;
+        deg0[x] = dx;
+    }
 }
 
 __global__ void __launch_bounds__(kMergeThreads) k_merge_tails(int n, const int32_t* __restrict__ iu,
@@ -338,20 +457,11 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge_tails_group(const __gri
 {
     const GraphBatchSlot& b = S.slot[blockIdx.y];
     const int e = blockIdx.x;
+    if (S.errs && e == 0 && threadIdx.x == 0) S.errs[blockIdx.y] = *b.err;
     if (e >= 2 * b.n) return;
     const int i = e < b.n ? e : e - b.n;
     if (b.ok[i] <= 0) return;
     merge_tail(b.row, b.deg, b.deg0, b.nsort, b.col, e < b.n ? b.iu[i] : b.iv[i]);
-}
-
-// After a batch: every appended slot becomes visible to all later traversals.
-__global__ void k_seal(int n, const int32_t* __restrict__ iu, const int32_t* __restrict__ iv,
-                       const int32_t* __restrict__ ok, const int32_t* __restrict__ deg, int32_t* deg0)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || ok[i] <= 0) return;
-    deg0[iu[i]] = deg[iu[i]];
-    deg0[iv[i]] = deg[iv[i]];
 }
 
 // Removes neighbour y from x's slots (one warp): the slot is found, the later
@@ -423,24 +533,6 @@ __global__ void k_remove(int64_t nv, const int64_t* __restrict__ row, int32_t* d
 // first of them, and in an unsorted tail (lists longer than one batch's merge)
 // the nth match is.  By one thread in order, each of its two binary searches a
 // chain of dependent loads, a batch of 256 on R-MAT 20 took 1.7 ms.
-
-// First slot of x in [0, ns) whose neighbour is >= y, 32 probes a step.
-__device__ __forceinline__ int warp_lower_bound(const int32_t* __restrict__ col, int64_t rx, int ns, int y)
-{
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    int lo = 0, hi = ns;
-    while (hi > lo) {
-        const int step = (hi - lo + 31) >> 5;
-        const int64_t p = lo + (int64_t)lane * step;
-        const int below = __popc(__ballot_sync(full, p < hi && col[rx + p] < y));  // probes ascend: the first `below`
-        const int base = lo;
-        if (below == 0) return base;
-        lo = (int)min((int64_t)hi, base + (int64_t)(below - 1) * step + 1);
-        hi = (int)min((int64_t)hi, base + (int64_t)below * step);
-    }
-    return lo;
-}
 
 // The slot of x that the deletion with `nth` earlier ones of its edge removes, or -1.
 __device__ __forceinline__ int64_t nth_slot(const int64_t* __restrict__ row, const int32_t* __restrict__ deg,
@@ -549,17 +641,6 @@ __global__ void __launch_bounds__(256) k_compact_removed(const int64_t* __restri
     }
 }
 
-// k_seal over many graphs: blockIdx.y selects the graph.
-__global__ void k_seal_group(const __grid_constant__ GraphBatchSlots S)
-{
-    const GraphBatchSlot& b = S.slot[blockIdx.y];
-    if (S.errs && blockIdx.x == 0 && threadIdx.x == 0) S.errs[blockIdx.y] = *b.err;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= b.n || b.ok[i] <= 0) return;
-    b.deg0[b.iu[i]] = b.deg[b.iu[i]];
-    b.deg0[b.iv[i]] = b.deg[b.iv[i]];
-}
-
 // Copy every vertex's live slots to a new layout with larger slack (warp per vertex).
 __global__ void k_repack(int64_t nv, const int64_t* __restrict__ orow, const int32_t* __restrict__ deg,
                          const int32_t* __restrict__ ocol, const int32_t* __restrict__ oseq,
@@ -590,6 +671,12 @@ cudaError_t launch_append(sbc_graph* g, int n, bool directed)
                                           directed ? 1 : 0, g->d_err);
         return cudaGetLastError();
     }
+    if (n <= kFusedAppendMax) {
+        k_append_small<<<1, 32 * std::min(n, 32), 0, g->stream>>>(g->nv, g->d_row, g->d_deg, g->d_deg0, g->d_nsort,
+                                                                  g->d_cap, g->d_col, g->d_seq, n, iu, iv, ok,
+                                                                  directed ? 1 : 0, g->d_err);
+        return cudaGetLastError();
+    }
     int32_t* rk = g->d_ins + 3 * g->ins_capacity;
     const int wblocks = (n + 7) / 8;  // 8 warps of 32 per block, a warp per insertion
     k_append_codes<<<wblocks, 256, 0, g->stream>>>(g->nv, g->d_row, g->d_deg, g->d_nsort, g->d_col, n, iu, iv, ok,
@@ -608,7 +695,6 @@ cudaError_t launch_seal(sbc_graph* g, int n)
     if (n <= 0) return cudaSuccess;
     k_merge_tails<<<2 * n, kMergeThreads, 0, g->stream>>>(n, iu, iv, ok, g->d_row, g->d_deg, g->d_deg0, g->d_nsort,
                                                           g->d_col);
-    k_seal<<<(n + 255) / 256, 256, 0, g->stream>>>(n, iu, iv, ok, g->d_deg, g->d_deg0);
     cudaError_t e = cudaGetLastError();
     if (e) return e;
     return launch_l2mask_insert(g, n, g->last_directed);
@@ -636,7 +722,9 @@ GraphBatchSlot graph_batch_slot(sbc_graph* g, int n)
 cudaError_t launch_append_group(const GraphBatchSlots& S, cudaStream_t s)
 {
     if (S.count <= 0) return cudaSuccess;
-    k_append_group<<<S.count, 32, 0, s>>>(S);
+    int nmax = 0;
+    for (int i = 0; i < S.count; ++i) nmax = std::max(nmax, S.slot[i].n);
+    k_append_group<<<S.count, 32 * std::min(std::max(nmax, 1), 32), 0, s>>>(S);
     return cudaGetLastError();
 }
 
@@ -646,7 +734,6 @@ cudaError_t launch_seal_group(const GraphBatchSlots& S, cudaStream_t s)
     for (int i = 0; i < S.count; ++i) nmax = std::max(nmax, S.slot[i].n);
     if (S.count <= 0 || nmax <= 0) return cudaSuccess;
     k_merge_tails_group<<<dim3(2 * nmax, S.count), kMergeThreads, 0, s>>>(S);
-    k_seal_group<<<dim3((nmax + 255) / 256, S.count), 256, 0, s>>>(S);
     return cudaGetLastError();
 }
 

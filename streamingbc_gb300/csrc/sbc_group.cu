@@ -4,7 +4,7 @@
 // The reference updates one forest per insertEdgeStreamingBC call
 // (src/streamingbc.c:88-226); a caller with many small graphs pays one full
 // pass of launches per graph and leaves most SMs idle on each.  Here a group
-// stages every member's insertions, appends them all in one launch (one warp
+// stages every member's insertions, appends them all in one launch (one CTA
 // per graph, k_append_group), culls roots of all members in one classify
 // launch, and runs one persistent update launch whose work items are
 // (member, root) pairs drawn from a single queue, so large and small graphs
