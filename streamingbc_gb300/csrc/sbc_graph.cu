@@ -590,9 +590,11 @@ __global__ void k_mark_removed(const int64_t* __restrict__ row, const int32_t* _
 // Batched deletions, step 3 (after the update): the marked slots leave their
 // lists, which keep their order.  CTA per deletion endpoint; the first CTA to
 // reach a vertex claims it by swapping its deg0 (== deg between batches) for
-// -1 until it is done, and CTAs that find it claimed leave it (one arriving
-// after the claimer finished compacts a clean list again, which changes
-// nothing).
+// -1, and CTAs that find it claimed leave it.  The claim outlives the launch
+// (k_reopen ends it): a CTA that came after a claim was given up would read
+// the vertex's degree and slots as its own SM last cached them, and put slots
+// back that had left the list.  A single deletion has two endpoints and no
+// second comer, so its CTAs end their claims themselves.
 __global__ void __launch_bounds__(256) k_compact_removed(const int64_t* __restrict__ row, int32_t* deg, int32_t* deg0,
                                                          int32_t* nsort, int32_t* col, int32_t* seq, int n,
                                                          const int32_t* __restrict__ iu,
@@ -605,10 +607,7 @@ __global__ void __launch_bounds__(256) k_compact_removed(const int64_t* __restri
     const int i = blockIdx.x >> 1;
     if (code[i] != 1) return;
     const int x = (blockIdx.x & 1) ? iv[i] : iu[i];
-    if (threadIdx.x == 0) {
-        const int d0 = deg0[x];
-        s_mine = d0 >= 0 && atomicCAS(&deg0[x], d0, -1) == d0;
-    }
+    if (threadIdx.x == 0) s_mine = atomicExch(&deg0[x], -1) >= 0;
     __syncthreads();
     if (!s_mine) return;
     const int64_t rx = row[x];
@@ -636,9 +635,19 @@ __global__ void __launch_bounds__(256) k_compact_removed(const int64_t* __restri
     }
     if (threadIdx.x == 0) {
         deg[x] = kept;
-        deg0[x] = kept;
+        if (n == 1) deg0[x] = kept;
         nsort[x] = s_keep_sorted;
     }
+}
+
+// Ends the claims of k_compact_removed.
+__global__ void k_reopen(const int32_t* __restrict__ deg, int32_t* deg0, int n, const int32_t* __restrict__ iu,
+                         const int32_t* __restrict__ iv, const int32_t* __restrict__ code)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n || code[i] != 1) return;
+    deg0[iu[i]] = deg[iu[i]];
+    deg0[iv[i]] = deg[iv[i]];
 }
 
 // Copy every vertex's live slots to a new layout with larger slack (warp per vertex).
@@ -762,6 +771,11 @@ cudaError_t launch_compact_removed(sbc_graph* g, int n)
                                                     g->d_ins + 2 * g->ins_capacity);
     cudaError_t e = cudaGetLastError();
     if (e) return e;
+    if (n > 1) {
+        k_reopen<<<(n + 255) / 256, 256, 0, g->stream>>>(g->d_deg, g->d_deg0, n, g->d_ins, g->d_ins + g->ins_capacity,
+                                                         g->d_ins + 2 * g->ins_capacity);
+        if ((e = cudaGetLastError())) return e;
+    }
     return launch_l2mask_remove_batch(g, n);
 }
 
