@@ -1065,10 +1065,15 @@ StaticShape static_shape(int64_t nv, int64_t nk, int64_t workers, int sm_count, 
     return S;
 }
 
-cudaError_t static_launch(const StaticShape& S, const StaticArgs& A, cudaStream_t s)
+// The shared-memory limit belongs to the kernel, not to the launch, and host
+// threads with graphs of different sizes share it: every call sets the same
+// value, all that a CTA of this kernel can have, so that none lowers it between
+// another's setting and launch.
+cudaError_t static_launch(const StaticShape& S, const StaticArgs& A, size_t smem_block, cudaStream_t s)
 {
     if (S.dyn + static_fixed(S.nt, S.mode) > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(S.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.dyn);
+        const int most = (int)(smem_block - static_fixed(S.nt, S.mode) - 1024);
+        cudaError_t e = cudaFuncSetAttribute(S.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         if (e) return e;
     }
     S.kernel<<<S.grid, S.nt, S.dyn, s>>>(A);
@@ -1125,7 +1130,7 @@ cudaError_t launch_static_list(sbc_forest* f, const int* d_list, const int* d_nl
     A.halves = S.halves;
     A.third_bits = 0;
     f->prof_begin(PROF_STATIC);
-    e = static_launch(S, A, s);
+    e = static_launch(S, A, smem_block, s);
     f->prof_end(PROF_STATIC);
     if (e) return e;
     if (d_list) return cudaSuccess;  // the caller moves BC by the listed roots' old and new rows
@@ -1339,7 +1344,7 @@ extern "C" int sbc_static_init_noalloc(int64_t nv, const int64_t* d_off, const i
     if (S.mode > kBits) return noalloc_fail(SBC_ERR_CUDA, "sbc_static_init_noalloc: too little shared memory");
     A.halves = 1;
     A.third_bits = S.mode == kBits;
-    if (static_launch(S, A, s) != cudaSuccess)
+    if (static_launch(S, A, smem_block, s) != cudaSuccess)
         return noalloc_fail(SBC_ERR_CUDA, "sbc_static_init_noalloc: k_static launch failed");
     if (launch_bc_colsum(d_delta, d_roots, (int)nk, nv, d_bc, bad, s) != cudaSuccess)
         return noalloc_fail(SBC_ERR_CUDA, "sbc_static_init_noalloc: k_bc_colsum launch failed");
