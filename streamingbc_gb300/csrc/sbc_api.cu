@@ -132,6 +132,9 @@ int repack(sbc_graph* g, const std::unordered_map<int64_t, int64_t>& need)
     g->h_row = row;
     g->h_cap = cap;
     for (int64_t v = 0; v < g->nv; ++v) g->h_deg_ub[v] = deg[v];
+    std::fill(g->h_freed.begin(), g->h_freed.end(), 0);
+    g->reserved = 0;
+    g->unreserved = false;
     g->repacks++;
     return SBC_OK;
 }
@@ -140,16 +143,25 @@ int repack(sbc_graph* g, const std::unordered_map<int64_t, int64_t>& need)
 // counts them into the host degree upper bound.
 int plan_capacity(sbc_graph* g, int64_t n, const int64_t* u, const int64_t* v, bool directed)
 {
+    if (g->unreserved) {
+        // what device batches beyond the reservations took from the slack
+        CK(cudaStreamSynchronize(g->stream));
+        std::vector<int32_t> deg(g->nv);
+        if (g->nv) CK(cudaMemcpy(deg.data(), g->d_deg, sizeof(int32_t) * g->nv, cudaMemcpyDeviceToHost));
+        for (int64_t v = 0; v < g->nv; ++v) g->h_deg_ub[v] = std::max<int64_t>(g->h_deg_ub[v], deg[v]);
+        std::fill(g->h_freed.begin(), g->h_freed.end(), 0);
+        g->unreserved = false;
+    }
     std::unordered_map<int64_t, int64_t> need;
     bool over = false;
     for (int64_t i = 0; i < n; ++i) {
         const int64_t a = u[i], b = v[i];
         if (a == b || a < 0 || b < 0 || a >= g->nv || b >= g->nv) continue;
         int64_t na = ++need[a];
-        if (g->h_deg_ub[a] + na > g->h_cap[a]) over = true;
+        if (g->deg_bound(a) + na > g->h_cap[a]) over = true;
         if (!directed) {
             int64_t nb = ++need[b];
-            if (g->h_deg_ub[b] + nb > g->h_cap[b]) over = true;
+            if (g->deg_bound(b) + nb > g->h_cap[b]) over = true;
         }
     }
     if (over) {
@@ -638,6 +650,7 @@ int sbc_graph_create(sbc_graph** out, int64_t nv, const int64_t* off, const int6
     g->h_row.resize(nv + 1);
     g->h_cap.resize(nv);
     g->h_deg_ub.resize(nv);
+    g->h_freed.assign(nv, 0);
     std::vector<int32_t> deg(nv);
     int64_t total = 0;
     for (int64_t v = 0; v < nv; ++v) {
@@ -760,7 +773,11 @@ int sbc_graph_reserve(sbc_graph* g, int64_t n, const int64_t* u, const int64_t* 
 {
     if (!g || n < 0 || (n > 0 && (!u || !v))) return fail(SBC_ERR_ARG, "sbc_graph_reserve: bad arguments");
     if (use_device(g->device)) return SBC_ERR_CUDA;
-    return plan_capacity(g, n, u, v, false);
+    const int rc = plan_capacity(g, n, u, v, false);
+    if (rc) return rc;
+    for (int64_t i = 0; i < n; ++i)
+        if (u[i] != v[i] && u[i] >= 0 && v[i] >= 0 && u[i] < g->nv && v[i] < g->nv) g->reserved++;
+    return SBC_OK;
 }
 
 int sbc_graph_repacks(const sbc_graph* g, int64_t* count)
@@ -818,7 +835,7 @@ int sbc_forest_create_ex(sbc_forest** out, sbc_graph* g, int64_t nk, const int64
     if (variant < 0) {
         const char* env = getenv("SBC_UPDATE_VARIANT");
         int64_t slots = 0;
-        for (int64_t d : g->h_deg_ub) slots += d;
+        for (int64_t v = 0; v < g->nv; ++v) slots += g->deg_bound(v);
         variant = env ? atoi(env) : sbc::update_variant_for(slots);
     }
     if (variant < 0 || variant >= sbc::update_variant_count())
@@ -1027,6 +1044,8 @@ int sbc_insert_batch_device(sbc_forest* f, int64_t n, const int32_t* d_u, const 
     int rc = ensure_staging(g, n);
     if (rc) return rc;
     if ((rc = ensure_model_batch(f, g->ins_capacity))) return rc;
+    if (n > g->reserved) g->unreserved = true;
+    g->reserved -= std::min<int64_t>(n, g->reserved);
     if (f->use_graphs && !f->prof) return replay_batch(f, (int)n, d_u, d_v);
     f->prof_begin(sbc::PROF_BATCH);
     CK(sbc::launch_set_src(g, d_u, d_v));
@@ -1213,7 +1232,7 @@ int sbc_graph_remove_directed(sbc_graph* g, int64_t from, int64_t to, int* resul
     CK(cudaStreamSynchronize(g->stream));
     if (*result == 1) {
         g->edge_skew -= sbc::edge_mix((int)from, (int)to);
-        g->h_deg_ub[from]--;
+        g->h_freed[from]++;
     }
     return SBC_OK;
 }
@@ -1249,8 +1268,8 @@ int sbc_delete_batch(sbc_forest* f, int64_t n, const int64_t* u, const int64_t* 
     const int32_t* codes = g->h_codes();
     for (int64_t i = 0; i < n; ++i)
         if (codes[i] > 0) {
-            g->h_deg_ub[u[i]]--;
-            g->h_deg_ub[v[i]]--;
+            g->h_freed[u[i]]++;
+            g->h_freed[v[i]]++;
         }
     if (stats) fill_stats(g, n, R->counters, stats);
     if (R->dirty > 0) {

@@ -144,7 +144,16 @@ struct sbc_graph {
     // host mirrors used to plan re-packs without reading the device
     std::vector<int64_t> h_row;
     std::vector<int32_t> h_cap;
-    std::vector<int64_t> h_deg_ub;  // upper bound of the live degree
+    // Upper bound of the live degree: exact after a re-pack, raised by every
+    // insertion that the host knows or was asked to reserve for.  Removals are
+    // counted apart, in h_freed, and taken off only while every device batch
+    // was reserved for: the slack also takes batches that were not, and those
+    // are in no bound until the next planned batch reads the degrees.
+    std::vector<int64_t> h_deg_ub;
+    std::vector<int64_t> h_freed;
+    int64_t reserved = 0;     // pairs reserved that no device batch has used yet
+    bool unreserved = false;  // a device batch went beyond what was reserved since the degrees were read
+    int64_t deg_bound(int64_t v) const { return h_deg_ub[v] - (unreserved ? 0 : h_freed[v]); }
     // staging for insertion batches
     int ins_capacity = 0;
     int32_t* d_ins = nullptr;  // [5 * ins_capacity + 1]: u, v, ok, then the append's ranks and misfit flag
