@@ -116,8 +116,8 @@ int sbc_graph_create_dimacs(sbc_graph **out, const char *path, int64_t *nv, int6
  * persistent CTAs are sized from occupancy and free memory (0 = automatic). */
 int sbc_forest_create(sbc_forest **out, sbc_graph *g, int64_t nk, const int64_t *roots, int64_t workers);
 /* As sbc_forest_create with an explicit launch shape of the update kernel
- * (variant -1: the SBC_UPDATE_VARIANT environment variable, else by the size of
- * the graph's adjacency). */
+ * (variant -1: the SBC_UPDATE_VARIANT environment variable, else by the number
+ * of roots and the size of the graph). */
 int sbc_forest_create_ex(sbc_forest **out, sbc_graph *g, int64_t nk, const int64_t *roots, int64_t workers,
                          int variant);
 /* Launch shapes of the update kernel in this build: threads per CTA and the

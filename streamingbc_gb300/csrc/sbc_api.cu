@@ -836,7 +836,9 @@ int sbc_forest_create_ex(sbc_forest** out, sbc_graph* g, int64_t nk, const int64
         const char* env = getenv("SBC_UPDATE_VARIANT");
         int64_t slots = 0;
         for (int64_t v = 0; v < g->nv; ++v) slots += g->deg_bound(v);
-        variant = env ? atoi(env) : sbc::update_variant_for(slots);
+        int sms = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device);
+        variant = env ? atoi(env) : sbc::update_variant_for(g->nv, slots, nk, std::max(sms, 1));
     }
     if (variant < 0 || variant >= sbc::update_variant_count())
         return fail(SBC_ERR_ARG, "update variant %d out of range", variant);

@@ -400,8 +400,9 @@ inline ForestSlot forest_slot(const sbc_forest* f, int n)
 
 int update_variant_count();
 int update_default_variant();
-// The update shape of a forest created without one, on a graph of that many adjacency slots.
-int update_variant_for(int64_t slots);
+// The update shape of a forest of nk roots created without one, on a graph of
+// nv vertices and that many adjacency slots.
+int update_variant_for(int64_t nv, int64_t slots, int64_t nk, int sm_count);
 int update_variant_threads(int v);
 int update_workers_per_sm(int v);
 // Sets the calling thread's sbc_last_error() message and returns code.

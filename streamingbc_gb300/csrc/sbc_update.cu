@@ -209,27 +209,43 @@ static const UpdateVariant kVariants[] = {
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 constexpr int kDefaultVariant = 7;  // 1024 threads, one root per SM
 
-// The shape of a forest created without one, by the adjacency slots of its
-// graph (what a root's walks can scan).  Measured, insert / delete of a batch in
-// us, 128x8 (2 slots in flight) | 256x4 (2) | 512x2 | 1024x1:
-//   ER 1024 K=1024, 16 k slots         1431/912 | 1606/965 | 2474/1261 | 4075/1948
-//   ER 4000 K=500, 40 k                1238/1008 | 960/1019 | 1230/1081 | 1945/1344
-//   Chung-Lu 5k K=400, 50 k            1079/1079 | 856/1058 | 907/1083 | 1337/1341
-//   R-MAT 13 K=300, 131 k              1017/1192 | 792/1007 | 742/927 | 854/973
-//   Chung-Lu 40k K=256, 352 k          2205/2498 | 1687/1851 | 1623/1709 | 2306/2719
-//   Chung-Lu 100k K=300, 1.2 M         3462/3961 | 2249/2384 | 1958/2080 | 2400/2980
-//   R-MAT 16 K=300, 2 M                2202/2767 | 1488/1533 | 1056/1196 | 1027/1486
-//   R-MAT 17 K=301, 4 M                4035/4439 | 2350/2630 | 1571/1742 | 1332/1752
-//   R-MAT 19 K=300, 16 M               18587/25045 | 10589/11998 | 6358/7294 | 5067/5179
-// Small graphs are bound by the latency of a job's steps, so more roots in
-// flight; from about 1.5 M slots on the walks of a job are, so the whole SM on
-// one root (and its gathered rows stay in L2).
-int update_variant_for(int64_t slots)
+// The shape of a forest created without one: by the CTAs per SM that its roots
+// fill, the adjacency slots that a root's walks can scan, and the vertices that
+// a worker's scratch holds.  Measured, insert + delete of a batch of 64 in us
+// (70 % of the edges between near vertices, R-MAT's drawn by R-MAT), 128x8 (2
+// slots in flight) | 256x4 (2) | 512x2 | 512x1 | 1024x1:
+//   ER 4000, 40 k slots     K=152  2811 |  2464 |  2372 |  2192 |  2507
+//                           K=256  2915 |  2538 |  2519 |  2972 |  3430
+//                           K=500  3495 |  3091 |  3733 |  4606 |  5459
+//   ER 1024, 16 k           K=1024 2343 |  2571 |  3735 |     - |  6023
+//   R-MAT 14, 222 k         K=152  3413 |  2416 |  1982 |  1851 |  1951
+//                           K=500  5278 |  3778 |  3065 |  3286 |  3582
+//   Chung-Lu 40k, 352 k     K=152 10142 |  6362 |  4626 |  4387 |  4167
+//                           K=256  9070 |  5836 |  4410 |  5395 |  5659
+//                           K=500  9013 |  6175 |  5895 |  7927 |  8989
+//   ER 50k, 600 k           K=152 12895 |  7999 |  5623 |  5357 |  4863
+//                           K=256 16081 |  9685 |  6712 |  7258 |  6844
+//                           K=500 17867 | 11222 |  8960 | 11044 | 10833
+//   Chung-Lu 100k, 1.2 M    K=152 11229 |  6765 |  4701 |  4438 |  4085
+//                           K=256 22302 | 12732 |  8124 |  8285 |  6793
+//                           K=500 23276 | 13473 |  9318 | 10234 |  9592
+//   R-MAT 17, 3.6 M         K=152 20394 | 10672 |  6225 |  5868 |  4562
+//                           K=500 61992 | 31869 | 18096 | 17786 | 13276
+// Small graphs are bound by the latency of a job's steps, so as many roots in
+// flight as there are, and a CTA no narrower than they need; from about 0.5 M
+// slots on the walks of a job are, so the whole SM on one root (and its gathered
+// rows stay in L2), the more so where a batch has few jobs (8 uniform edges on
+// ER 50k, K=256: 1722 with 512x2, 1432 with 1024x1).  A graph of fewer than 4
+// slots a vertex counts as one of 4, so that many workers are not given the
+// scratch of many vertices.
+int update_variant_for(int64_t nv, int64_t slots, int64_t nk, int sm_count)
 {
-    if (slots < 24000) return 12;      // 128 x 8
-    if (slots < 100000) return 13;     // 256 x 4
-    if (slots < 1500000) return 5;     // 512 x 2
-    return kDefaultVariant;
+    slots = std::max<int64_t>(slots, 4 * nv);
+    const int64_t per_sm = (nk + sm_count - 1) / sm_count;
+    if (slots >= 500000) return kDefaultVariant;           // 1024 x 1
+    if (per_sm <= 1) return 6;                             // 512 x 1
+    if (per_sm <= 2 || slots >= 100000) return 5;          // 512 x 2
+    return per_sm <= 4 || slots >= 24000 ? 13 : 12;        // 256 x 4, 128 x 8
 }
 
 // Deletion of (u, v), already removed from the adjacency: warp per root.  A
