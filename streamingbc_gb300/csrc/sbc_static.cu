@@ -66,15 +66,32 @@ constexpr int kSlotLevels = 64;   // levels whose slot counts the backward pass 
 constexpr int kLaneSlots = 8;
 constexpr int kBigDeg = 1024;
 constexpr int kSegSlots = 2048;
-// Such vertices listed per walk (the others stay a warp's).
+// The backward pass pushes only into vertices of fewer neighbours than 1/16 of
+// the graph's largest number, within these bounds: pushed weights are added one
+// after the other, and into one address one at a time, while a pull sums a long
+// list with 32 lanes a segment.  Largest error of a dependency against long
+// double with pulls of a warp alone | pushes into any vertex | this rule:
+//   R-MAT 18, 16 roots       2.9e-15 | 3.6e-14 | 1.9e-15
+//   R-MAT 20, 8              2.9e-15 | 4.4e-14 | 2.6e-15
+//   Chung-Lu 40k, 64         9.2e-16 | 1.3e-15 | 6.8e-16
+//   5 hubs, 100k leaves, 16  1.4e-14 | 1.9e-12 | 9.5e-16
+// Without the lower bound Chung-Lu (degrees to 300) would scan a third more
+// slots; 1/8 puts R-MAT 18 at 4.1e-15.  The time of the two last forms: R-MAT
+// 18, 251 roots 9.4 | 10.7 ms, R-MAT 20, 304 roots 44.4 | 46.3 ms, Chung-Lu
+// 40k, 256 roots 1.15 | 1.22 ms; a star of 5,000, 300 roots 1.41 | 0.18 ms.
+constexpr int kPushDegMin = 128, kPushDegMax = 4096, kPushDegPart = 16;
+constexpr int kLongShift = 40;
+// Vertices of kBigDeg or more listed per walk (the others stay a warp's).
 constexpr int kBigCap = 1024, kBigCapSmall = 64;
 
 template <int NT, int CAP>
 struct StaticSmem {
     static constexpr int kCap = CAP;
     int item, tail, next, next_seg, nbig;
-    unsigned long long slots, total;
-    unsigned long long lvslots[kSlotLevels];
+    unsigned max_deg;
+    unsigned long long slots, long_slots, total;
+    unsigned long long lvslots[kSlotLevels];  // of each level's vertices
+    unsigned long long lvlong[kSlotLevels];   // of those too long to push into; their number from bit kLongShift on
     int big[CAP];
     int seg_end[CAP];  // running segment counts of big[]
     unsigned char bighit[CAP];
@@ -469,8 +486,9 @@ __device__ __forceinline__ void unset_tasks(const DevGraph& G, Sm& sm, const uin
 //     one-byte distance row cost an L2 sector per scanned slot.
 //   * Each pair of levels is walked from its cheaper side: forward, the frontier
 //     pushes or, when fewer slots are left, the unvisited vertices pull;
-//     backward, the parents pull or the children push.  On R-MAT graphs the
-//     hubs sit on the middle levels, and 2.4 times fewer slots are scanned.
+//     backward, the parents pull or, short lists alone (kPushDegMin), the
+//     children push.  On R-MAT graphs the hubs sit on the middle levels, and
+//     about three times fewer slots are scanned.
 //   * Warps take vertices from the level by themselves (list_tasks): three
 //     block barriers per level instead of five per 1,024 vertices, and the
 //     counters come from the level sizes instead of shared atomics.
@@ -539,6 +557,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
         if (threadIdx.x == 0) {
             sm.item = atomicAdd(A.work_counter, 1);
             sm.total = 0;
+            sm.max_deg = 0;
         }
         __syncthreads();
         const int item = sm.item;
@@ -558,6 +577,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
 
         {
             unsigned long long sum = 0;
+            unsigned most = 0;
             for (int64_t x = threadIdx.x; x < (int64_t)nw * 32; x += NT) {
                 int d = 0;
                 if (x < nv) {
@@ -567,15 +587,21 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                     if (MODE == kSmall) acc[x] = 0.0;
                 }
                 sum += (unsigned)d;
+                most = max(most, (unsigned)d);
                 const unsigned word = __ballot_sync(full, x >= nv || (sym && d == 0));
                 if (lane == 0) V[x >> 5] = word;
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(full, sum, o);
-            if (lane == 0) atomicAdd(&sm.total, sum);
+            most = __reduce_max_sync(full, most);
+            if (lane == 0) {
+                atomicAdd(&sm.total, sum);
+                atomicMax(&sm.max_deg, most);
+            }
         }
         __syncthreads();
         const unsigned long long total = sm.total;
+        auto push_deg = [&]() { return min(max((int)(sm.max_deg / kPushDegPart), kPushDegMin), kPushDegMax); };
         int nlev = 0, reached = 0;
         unsigned long long visited = 0, scanned = 0;
         if (valid) {
@@ -587,6 +613,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                 lvl[0] = 0;
                 sm.tail = 1;
                 sm.lvslots[0] = front;
+                sm.lvlong[0] = (int)front >= push_deg() ? front + (1ull << kLongShift) : 0ull;
                 V[root >> 5] |= 1u << (root & 31);
             }
             visited = front;
@@ -603,7 +630,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                 uint32_t* const N = pull ? Npull : Npush;
                 if (threadIdx.x == 0) sm.next = sm.nbig = 0;
                 __syncthreads();
-                if (threadIdx.x == 0) sm.slots = 0;
+                if (threadIdx.x == 0) sm.slots = sm.long_slots = 0;
                 if (!pull) {
                     scanned += front;
                     const uint32_t* T = MODE == kOneBits ? B : V;
@@ -697,7 +724,12 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                 // B and N are empty again between levels (or B is the visited set)
                 if (pull)
                     for (int i = lo + threadIdx.x; i < hi; i += NT) B[qd[i] >> 5] = 0u;
-                unsigned long long sum = 0;
+                unsigned long long sum = 0, longs = 0;
+                auto count = [&](int x) {
+                    const unsigned d = (unsigned)A.G.deg[x];
+                    sum += d;
+                    if ((int)d >= push_deg()) longs += d + (1ull << kLongShift);
+                };
                 lo = hi;
                 if (dense) {
                     // N listed in vertex order, added to the visited set and
@@ -727,7 +759,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                                 const int x = (i0 + j) * 32 + lane;
                                 qd[pos + __popc(w & ((1u << lane) - 1u))] = x;
                                 D[x] = L + 1;
-                                sum += (unsigned)A.G.deg[x];
+                                count(x);
                             }
                             pos += __popc(w);
                         }
@@ -741,7 +773,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                         atomicOr(&V[x >> 5], bit);
                         if (MODE == kOneBits && held) atomicOr(&B[x >> 5], bit);
                         N[x >> 5] = 0u;
-                        sum += (unsigned)A.G.deg[x];
+                        count(x);
                     }
                 }
                 if (lo == hi) break;
@@ -749,11 +781,19 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(full, sum, o);
                 if (lane == 0 && sum) atomicAdd(&sm.slots, sum);
+                if (__any_sync(full, longs != 0)) {
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) longs += __shfl_xor_sync(full, longs, o);
+                    if (lane == 0) atomicAdd(&sm.long_slots, longs);
+                }
                 if (threadIdx.x == 0) lvl[L] = lo;
                 __syncthreads();
                 front = sm.slots;
                 visited += front;
-                if (threadIdx.x == 0 && L < kSlotLevels) sm.lvslots[L] = front;
+                if (threadIdx.x == 0 && L < kSlotLevels) {
+                    sm.lvslots[L] = front;
+                    sm.lvlong[L] = sm.long_slots;
+                }
             }
             nlev = L + 1;
             reached = hi;
@@ -769,45 +809,37 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                 acc[x] = child_weight(nd + 1.0, sw);
             };
             for (int i = lvl[nlev - 1] + threadIdx.x; i < reached; i += NT) finish(qd[i], 0.0);
+            if (threadIdx.x == 0) sm.next = sm.nbig = 0;
             __syncthreads();
             int end = reached;  // of level l + 1
             for (int l = nlev - 2; l >= 0; --l) {
                 const int a0 = lvl[l], a1 = lvl[l + 1];
-                const bool push = sym && l + 1 < kSlotLevels && sm.lvslots[l + 1] < sm.lvslots[l];
-                const int m0 = push ? a0 : a1, m1 = push ? a1 : end;  // the level in the bitmap
-                for (int i = m0 + threadIdx.x; i < m1; i += NT) atomicOr(&B[qd[i] >> 5], 1u << (qd[i] & 31));
-                if (threadIdx.x == 0) {
-                    sm.next = sm.nbig = 0;
-                    if (l + 1 < kSlotLevels) sm.scanned += push ? sm.lvslots[l + 1] : sm.lvslots[l];
-                }
-                __syncthreads();
-                if (push) {
-                    auto act = [&](double w, const int (&k)[kLaneSlots]) {
-                        const unsigned in = in_bitmap(B, k);
-#pragma unroll
-                        for (int u = 0; u < kLaneSlots; ++u)
-                            if ((in >> u) & 1u) atomicAdd(&acc[k[u]], w);
-                    };
-                    list_tasks<NT, double>(A.G, sm, qd + a1, end - a1, sm.lvslots[l + 1], [&](int x) { return acc[x]; },
-                                           [&](const TaskVertex<double>& q, bool) { push_batch(A.G, sm, q, act); });
-                    const int nb = big_segments(A.G, sm, [&](int, int x, int64_t rs, int s0, int s1) {
-                        const double w = acc[x];
-                        for (int i = s0 + lane; i < s1; i += 32 * kLaneSlots) {
-                            int k[kLaneSlots];
-                            load_slots(A.G, rs, s1, i, 32, k);
-                            act(w, k);
+                const unsigned long long longs = l < kSlotLevels ? sm.lvlong[l] : 0ull;
+                const unsigned long long long_slots = longs & ((1ull << kLongShift) - 1);
+                const bool push = sym && l + 1 < kSlotLevels && sm.lvslots[l + 1] + long_slots < sm.lvslots[l];
+                const bool part = push && longs != 0;  // long lists are pulled all the same
+                if (!push || part) {
+                    for (int i = a1 + threadIdx.x; i < end; i += NT) atomicOr(&B[qd[i] >> 5], 1u << (qd[i] & 31));
+                    // a few long lists: straight to big_segments
+                    const bool listed = part && longs >> kLongShift <= (unsigned)Sm::kCap;
+                    if (listed)
+                        for (int i = a0 + threadIdx.x; i < a1; i += NT) {
+                            const int x = qd[i];
+                            if (A.G.deg[x] >= push_deg()) sm.big[atomicAdd(&sm.nbig, 1)] = x;
                         }
-                        __syncwarp();
-                    });
-                    if (nb > 0) __syncthreads();
-                    for (int i = a0 + threadIdx.x; i < a1; i += NT) finish(qd[i], acc[qd[i]]);
-                } else {
-                    list_tasks<NT, int>(A.G, sm, qd + a0, a1 - a0, l < kSlotLevels ? sm.lvslots[l] : 0ull,
-                                        [](int) { return 0; },
-                                        [&](const TaskVertex<int>& q, bool ok) {
-                                            pull_batch<double>(A.G, sm, q, ok, B, acc,
+                    if (threadIdx.x == 0 && l + 1 < kSlotLevels) sm.scanned += part ? long_slots : sm.lvslots[l];
+                    __syncthreads();
+                    if (!listed)
+                        list_tasks<NT, int>(A.G, sm, qd + a0, a1 - a0, l < kSlotLevels ? sm.lvslots[l] : 0ull,
+                                            [](int) { return 0; },
+                                            [&](TaskVertex<int> q, bool ok) {
+                                                if (part && q.d < push_deg()) {
+                                                    q.d = 0;
+                                                    ok = false;
+                                                }
+                                                pull_batch<double>(A.G, sm, q, ok, B, acc,
                                                                    [&](int y, double sum, bool) { finish(y, sum); });
-                                        });
+                                            });
                     const int nb = big_segments(A.G, sm, [&](int, int x, int64_t rs, int s0, int s1) {
                         double s = 0.0;
                         unsigned any = 0;
@@ -826,10 +858,45 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                         __syncthreads();
                         for (int b = threadIdx.x; b < nb; b += NT) finish(sm.big[b], acc[sm.big[b]]);
                     }
+                    __syncthreads();
+                    for (int i = a1 + threadIdx.x; i < end; i += NT) B[qd[i] >> 5] = 0u;
+                    if (threadIdx.x == 0) sm.next = sm.nbig = 0;
+                    __syncthreads();
                 }
-                __syncthreads();
-                for (int i = m0 + threadIdx.x; i < m1; i += NT) B[qd[i] >> 5] = 0u;
-                __syncthreads();
+                if (push) {
+                    for (int i = a0 + threadIdx.x; i < a1; i += NT) {
+                        const int x = qd[i];
+                        if (!part || A.G.deg[x] < push_deg()) atomicOr(&B[x >> 5], 1u << (x & 31));
+                    }
+                    if (threadIdx.x == 0) sm.scanned += sm.lvslots[l + 1];
+                    __syncthreads();
+                    auto act = [&](double w, const int (&k)[kLaneSlots]) {
+                        const unsigned in = in_bitmap(B, k);
+#pragma unroll
+                        for (int u = 0; u < kLaneSlots; ++u)
+                            if ((in >> u) & 1u) atomicAdd(&acc[k[u]], w);
+                    };
+                    list_tasks<NT, double>(A.G, sm, qd + a1, end - a1, sm.lvslots[l + 1], [&](int x) { return acc[x]; },
+                                           [&](const TaskVertex<double>& q, bool) { push_batch(A.G, sm, q, act); });
+                    big_segments(A.G, sm, [&](int, int x, int64_t rs, int s0, int s1) {
+                        const double w = acc[x];
+                        for (int i = s0 + lane; i < s1; i += 32 * kLaneSlots) {
+                            int k[kLaneSlots];
+                            load_slots(A.G, rs, s1, i, 32, k);
+                            act(w, k);
+                        }
+                        __syncwarp();
+                    });
+                    __syncthreads();
+                    for (int i = a0 + threadIdx.x; i < a1; i += NT) {
+                        const int x = qd[i];
+                        if (bit_of(B, x)) finish(x, acc[x]);
+                    }
+                    __syncthreads();
+                    for (int i = a0 + threadIdx.x; i < a1; i += NT) B[qd[i] >> 5] = 0u;
+                    if (threadIdx.x == 0) sm.next = sm.nbig = 0;
+                    __syncthreads();
+                }
                 end = a1;
             }
         }
