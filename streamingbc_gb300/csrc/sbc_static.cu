@@ -63,7 +63,11 @@ constexpr int kSlotLevels = 64;   // levels whose slot counts the backward pass 
 // A vertex is scanned by one lane up to 8 neighbours, by 4 lanes up to 32, by
 // 16 up to 128 (each lane then has 8 at a time in flight), by the warp up to
 // kBigDeg, and beyond in segments of kSegSlots that the CTA's warps share out.
-constexpr int kLaneSlots = 8;
+// A task none of whose vertices has more than kFewSlots takes a shorter form of
+// the one-lane step: deep graphs are bound by the instructions of the few warps
+// that have work (a path of 20,000, one root 69.8 -> 59.4 ms; where whole rows
+// are in shared memory the test cost ER 1,024 as much as it gave paths).
+constexpr int kLaneSlots = 8, kFewSlots = 4;
 constexpr int kBigDeg = 1024;
 constexpr int kSegSlots = 2048;
 // The backward pass pushes only into vertices of fewer neighbours than 1/16 of
@@ -88,8 +92,9 @@ template <int NT, int CAP>
 struct StaticSmem {
     static constexpr int kCap = CAP;
     int item, tail, next, next_seg, nbig;
-    unsigned max_deg;
-    unsigned long long slots, long_slots, total;
+    int max_deg;
+    unsigned long long total;
+    unsigned long long slots[2], long_slots[2];  // of the level being listed, by its parity
     unsigned long long lvslots[kSlotLevels];  // of each level's vertices
     unsigned long long lvlong[kSlotLevels];   // of those too long to push into; their number from bit kLongShift on
     int big[CAP];
@@ -104,60 +109,63 @@ struct StaticSmem {
 __device__ __forceinline__ bool bit_of(const uint32_t* B, int k) { return (B[k >> 5] >> (k & 31)) & 1u; }
 
 // Neighbours s0, s0 + step, ... of a list of d slots at rs (-1 past its end).
-__device__ __forceinline__ void load_slots(const DevGraph& G, int64_t rs, int d, int s0, int step, int (&k)[kLaneSlots])
+template <int S>
+__device__ __forceinline__ void load_slots(const DevGraph& G, int64_t rs, int d, int s0, int step, int (&k)[S])
 {
 #pragma unroll
-    for (int u = 0; u < kLaneSlots; ++u) k[u] = s0 + step * u < d ? G.col[rs + s0 + step * u] : -1;
+    for (int u = 0; u < S; ++u) k[u] = s0 + step * u < d ? G.col[rs + s0 + step * u] : -1;
 }
 
 // Bit u: k[u] is a neighbour (>= 0) and in bitmap B.  All words are loaded
 // before any is tested.
-__device__ __forceinline__ unsigned in_bitmap(const uint32_t* B, const int (&k)[kLaneSlots])
+template <int S>
+__device__ __forceinline__ unsigned in_bitmap(const uint32_t* B, const int (&k)[S])
 {
-    unsigned w[kLaneSlots];
+    unsigned w[S];
 #pragma unroll
-    for (int u = 0; u < kLaneSlots; ++u) w[u] = B[max(k[u], 0) >> 5];
+    for (int u = 0; u < S; ++u) w[u] = B[max(k[u], 0) >> 5];
     unsigned in = 0;
 #pragma unroll
-    for (int u = 0; u < kLaneSlots; ++u) in |= (k[u] >= 0 ? (w[u] >> (k[u] & 31)) & 1u : 0u) << u;
+    for (int u = 0; u < S; ++u) in |= (k[u] >= 0 ? (w[u] >> (k[u] & 31)) & 1u : 0u) << u;
     return in;
 }
 
 // Bit u: k[u] is a neighbour.
-__device__ __forceinline__ unsigned present(const int (&k)[kLaneSlots])
+template <int S>
+__device__ __forceinline__ unsigned present(const int (&k)[S])
 {
     unsigned in = 0;
 #pragma unroll
-    for (int u = 0; u < kLaneSlots; ++u) in |= (k[u] >= 0 ? 1u : 0u) << u;
+    for (int u = 0; u < S; ++u) in |= (k[u] >= 0 ? 1u : 0u) << u;
     return in;
 }
 
 // s += val[k[u]] over the k[u] in bitmap B; returns their bits.  Every
 // neighbour is tested, then the values are gathered, then summed.
-template <class T>
-__device__ __forceinline__ unsigned sum_in(const uint32_t* B, const T* val, const int (&k)[kLaneSlots], T& s)
+template <class T, int S>
+__device__ __forceinline__ unsigned sum_in(const uint32_t* B, const T* val, const int (&k)[S], T& s)
 {
     const unsigned in = in_bitmap(B, k);
-    T y[kLaneSlots];
+    T y[S];
 #pragma unroll
-    for (int u = 0; u < kLaneSlots; ++u) y[u] = (in >> u) & 1u ? val[k[u]] : (T)0;
+    for (int u = 0; u < S; ++u) y[u] = (in >> u) & 1u ? val[k[u]] : (T)0;
 #pragma unroll
-    for (int u = 0; u < kLaneSlots; ++u)
+    for (int u = 0; u < S; ++u)
         if ((in >> u) & 1u) s += y[u];
     return in;
 }
 
 // Appends k[u] for every set bit u of each calling lane's `first`: the lanes
 // here reserve the queue's slots together.
-template <class Sm>
-__device__ __forceinline__ void append_first(Sm& sm, int32_t* q, const int (&k)[kLaneSlots], unsigned first)
+template <class Sm, int S>
+__device__ __forceinline__ void append_first(Sm& sm, int32_t* q, const int (&k)[S], unsigned first)
 {
     const unsigned act = __activemask();
     if (!__any_sync(act, first)) return;
     const unsigned below = (1u << (threadIdx.x & 31)) - 1u;
-    int total = 0, at[kLaneSlots];
+    int total = 0, at[S];
 #pragma unroll
-    for (int u = 0; u < kLaneSlots; ++u) {
+    for (int u = 0; u < S; ++u) {
         const unsigned m = __ballot_sync(act, (first >> u) & 1u);
         at[u] = total + __popc(m & below);
         total += __popc(m);
@@ -167,7 +175,7 @@ __device__ __forceinline__ void append_first(Sm& sm, int32_t* q, const int (&k)[
     if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(&sm.tail, total);
     base = __shfl_sync(act, base, leader);
 #pragma unroll
-    for (int u = 0; u < kLaneSlots; ++u)
+    for (int u = 0; u < S; ++u)
         if ((first >> u) & 1u) q[base + at[u]] = k[u];
 }
 
@@ -218,7 +226,7 @@ __device__ __forceinline__ void lane_groups(Sm& sm, const TaskVertex<V>& q, int 
 // (-1: none) of a vertex whose value is v, from whichever lane scans them.
 // Vertices of degree kBigDeg and more are listed for big_segments.  No block
 // barrier inside.
-template <class Sm, class V, class Act>
+template <bool FEW, class Sm, class V, class Act>
 __device__ __forceinline__ void push_batch(const DevGraph& G, Sm& sm, TaskVertex<V> q, Act act)
 {
     const unsigned full = 0xffffffffu;
@@ -230,12 +238,22 @@ __device__ __forceinline__ void push_batch(const DevGraph& G, Sm& sm, TaskVertex
             q.d = 0;
         }
     }
+    if (FEW && !__any_sync(full, q.d > kFewSlots)) {
+        int k[kFewSlots];
+        if (q.d > 0) {
+            load_slots(G, q.rs, q.d, 0, 1, k);
+            act(q.v, k);
+        }
+        __syncwarp();
+        return;
+    }
     int k[kLaneSlots];
     if (q.d > 0 && q.d <= kLaneSlots) {
         load_slots(G, q.rs, q.d, 0, 1, k);
         act(q.v, k);
     }
     __syncwarp();
+    if (!__any_sync(full, q.d > kLaneSlots)) return;
     lane_groups<4>(sm, q, kLaneSlots, 4 * kLaneSlots, [&](int j, int64_t rj, int dj, V vj, int) {
         if (j >= 0) {
             load_slots(G, rj, dj, lane & 3, 4, k);
@@ -266,7 +284,7 @@ __device__ __forceinline__ void push_batch(const DevGraph& G, Sm& sm, TaskVertex
 // One vertex per lane: sums val[k] over the neighbours k in bitmap B, the
 // lists shared out as in push_batch, and calls done(x, sum, whether any
 // neighbour passed) in the lane that brought x.
-template <class T, class Sm, class Done>
+template <bool FEW, class T, class Sm, class Done>
 __device__ __forceinline__ void pull_batch(const DevGraph& G, Sm& sm, TaskVertex<int> q, bool ok,
                                            const uint32_t* B, const T* val, Done done)
 {
@@ -281,10 +299,21 @@ __device__ __forceinline__ void pull_batch(const DevGraph& G, Sm& sm, TaskVertex
             ok = false;  // finished after big_segments
         }
     }
-    int k[kLaneSlots];
-    auto add = [&](T& s, bool& hit) { hit |= sum_in(B, val, k, s) != 0u; };
     T sum = (T)0;
     bool hit = false;
+    if (FEW && !__any_sync(full, q.d > kFewSlots)) {
+        int k[kFewSlots];
+        if (q.d > 0) {
+            load_slots(G, q.rs, q.d, 0, 1, k);
+            hit = sum_in(B, val, k, sum) != 0u;
+        }
+        __syncwarp();
+        if (ok) done(q.x, sum, hit);
+        __syncwarp();
+        return;
+    }
+    int k[kLaneSlots];
+    auto add = [&](T& s, bool& hit) { hit |= sum_in(B, val, k, s) != 0u; };
     if (q.d > 0 && q.d <= kLaneSlots) {
         load_slots(G, q.rs, q.d, 0, 1, k);
         add(sum, hit);
@@ -312,24 +341,26 @@ __device__ __forceinline__ void pull_batch(const DevGraph& G, Sm& sm, TaskVertex
             }
         });
     };
-    grouped(std::integral_constant<int, 4>(), kLaneSlots, 4 * kLaneSlots);
-    grouped(std::integral_constant<int, 16>(), 4 * kLaneSlots, 16 * kLaneSlots);
-    for (unsigned m = __ballot_sync(full, q.d > 16 * kLaneSlots); m; m &= m - 1) {
-        const int j = __ffs(m) - 1;
-        const int64_t rj = __shfl_sync(full, q.rs, j);
-        const int dj = __shfl_sync(full, q.d, j);
-        T s = (T)0;
-        bool h = false;
-        for (int s0 = lane; s0 < dj; s0 += 32 * kLaneSlots) {
-            load_slots(G, rj, dj, s0, 32, k);
-            add(s, h);
-        }
-        if (__any_sync(full, h)) {
+    if (__any_sync(full, q.d > kLaneSlots)) {
+        grouped(std::integral_constant<int, 4>(), kLaneSlots, 4 * kLaneSlots);
+        grouped(std::integral_constant<int, 16>(), 4 * kLaneSlots, 16 * kLaneSlots);
+        for (unsigned m = __ballot_sync(full, q.d > 16 * kLaneSlots); m; m &= m - 1) {
+            const int j = __ffs(m) - 1;
+            const int64_t rj = __shfl_sync(full, q.rs, j);
+            const int dj = __shfl_sync(full, q.d, j);
+            T s = (T)0;
+            bool h = false;
+            for (int s0 = lane; s0 < dj; s0 += 32 * kLaneSlots) {
+                load_slots(G, rj, dj, s0, 32, k);
+                add(s, h);
+            }
+            if (__any_sync(full, h)) {
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(full, s, o);
-            if (lane == j) {
-                sum = s;
-                hit = true;
+                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(full, s, o);
+                if (lane == j) {
+                    sum = s;
+                    hit = true;
+                }
             }
         }
     }
@@ -338,7 +369,7 @@ __device__ __forceinline__ void pull_batch(const DevGraph& G, Sm& sm, TaskVertex
 }
 
 // Vertices of a list, handed to the warps in tasks of up to 32 (fewer when the
-// list is short, so that every warp has work); batch(task vertex, ok) per
+// list is short, so that more warps have work); batch(task vertex, ok) per
 // warp.  The next task's slots and value(x) are loaded before the current one
 // is walked.
 template <int NT, class V, class Sm, class Value, class Batch>
@@ -346,14 +377,19 @@ __device__ __forceinline__ void list_tasks(const DevGraph& G, Sm& sm, const int3
                                            unsigned long long slots, Value value, Batch batch)
 {
     const int lane = threadIdx.x & 31;
-    int t = min(32, max(1, (n + NT / 32 - 1) / (NT / 32)));
+    // a few vertices of short lists are better off in a few warps: each warp
+    // that takes part costs a turn of the fp64 pipe and of the queue's counter
+    // (grid of 100 x 100, one root 1.78 ms with the level spread over all warps,
+    // 1.23 so)
+    const int least = slots > 64ull * n ? 1 : slots > 8ull * n ? 4 : 16;
+    int t = min(32, max(least, (n + NT / 32 - 1) / (NT / 32)));
     // about kSegSlots * 2 slots a task: lists come in vertex order, which
     // gathers the hubs of some graphs in a few tasks
     if (slots > 64ull * n) t = min(t, max(4, (int)(2ull * kSegSlots * n / slots)));
-    auto claim = [&](TaskVertex<V>& q, bool& ok) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(&sm.next, t);
-        base = __shfl_sync(0xffffffffu, base, 0);
+    // the first tasks go by warp number, the others by claims
+    const int given = t * (NT / 32);
+    int base = t * (int)(threadIdx.x >> 5);
+    auto take = [&](TaskVertex<V>& q, bool& ok) {
         ok = lane < t && base + lane < n;
         q.x = q.d = 0;
         q.rs = 0;
@@ -368,10 +404,15 @@ __device__ __forceinline__ void list_tasks(const DevGraph& G, Sm& sm, const int3
     };
     TaskVertex<V> q;
     bool ok;
-    for (bool more = claim(q, ok); more;) {
+    for (bool more = take(q, ok); more;) {
         TaskVertex<V> q2;
-        bool ok2;
-        more = claim(q2, ok2);
+        bool ok2 = false;
+        more = given < n;
+        if (more) {
+            if (lane == 0) base = given + atomicAdd(&sm.next, t);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            more = take(q2, ok2);
+        }
         batch(q, ok);
         q = q2;
         ok = ok2;
@@ -380,8 +421,9 @@ __device__ __forceinline__ void list_tasks(const DevGraph& G, Sm& sm, const int3
 
 // The walk's listed long vertices, a segment per warp at a time, once every
 // task is done: seg(i, x, rs, s0, s1) walks slots [s0, s1) of vertex x =
-// big[i].  Called by the whole CTA, with block barriers; returns how many
-// vertices are listed.
+// big[i].  Called by the whole CTA; returns how many vertices are listed, after
+// a block barrier that follows the tasks and, where that is not 0, one that
+// follows the segments.
 template <class Sm, class Seg>
 __device__ __forceinline__ int big_segments(const DevGraph& G, Sm& sm, Seg seg)
 {
@@ -421,6 +463,7 @@ __device__ __forceinline__ int big_segments(const DevGraph& G, Sm& sm, Seg seg)
         const int s0 = (u - (lo ? sm.seg_end[lo - 1] : 0)) * kSegSlots;
         seg(lo, x, G.row[x], s0, min(d, s0 + kSegSlots));
     }
+    __syncthreads();
     return nb;
 }
 
@@ -489,9 +532,10 @@ __device__ __forceinline__ void unset_tasks(const DevGraph& G, Sm& sm, const uin
 //     backward, the parents pull or, short lists alone (kPushDegMin), the
 //     children push.  On R-MAT graphs the hubs sit on the middle levels, and
 //     about three times fewer slots are scanned.
-//   * Warps take vertices from the level by themselves (list_tasks): three
-//     block barriers per level instead of five per 1,024 vertices, and the
-//     counters come from the level sizes instead of shared atomics.
+//   * Warps take vertices from the level by themselves (list_tasks): two block
+//     barriers per level on the way down and three on the way up instead of
+//     five per 1,024 vertices, and the counters come from the level sizes
+//     instead of shared atomics.
 //   * Levels, histogram and rosters leave the kernel with the rows.
 template <int NT, int MODE>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant__ StaticArgs A)
@@ -504,6 +548,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
     const int lane = threadIdx.x & 31;
     const int64_t nv = A.nv;
     const int nw = (int)((nv + 31) / 32);
+    constexpr bool kFew = MODE != kSmall;
     const bool sym = !A.asym && !(A.asym_dev && *A.asym_dev);
 
     // this worker's queue, level starts, child weights and bitmaps
@@ -577,7 +622,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
 
         {
             unsigned long long sum = 0;
-            unsigned most = 0;
+            int most = 0;
             for (int64_t x = threadIdx.x; x < (int64_t)nw * 32; x += NT) {
                 int d = 0;
                 if (x < nv) {
@@ -587,23 +632,19 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                     if (MODE == kSmall) acc[x] = 0.0;
                 }
                 sum += (unsigned)d;
-                most = max(most, (unsigned)d);
+                most = max(most, d);
                 const unsigned word = __ballot_sync(full, x >= nv || (sym && d == 0));
                 if (lane == 0) V[x >> 5] = word;
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(full, sum, o);
-            most = __reduce_max_sync(full, most);
-            if (lane == 0) {
-                atomicAdd(&sm.total, sum);
-                atomicMax(&sm.max_deg, most);
-            }
+            if (lane == 0) atomicAdd(&sm.total, sum);
+            if (most >= kPushDegMin) atomicMax(&sm.max_deg, most);
         }
         __syncthreads();
-        const unsigned long long total = sm.total;
-        auto push_deg = [&]() { return min(max((int)(sm.max_deg / kPushDegPart), kPushDegMin), kPushDegMax); };
+        auto push_deg = [&]() { return min(max(sm.max_deg / kPushDegPart, kPushDegMin), kPushDegMax); };
         int nlev = 0, reached = 0;
-        unsigned long long visited = 0, scanned = 0;
+        unsigned long long visited = 0;
         if (valid) {
             unsigned long long front = (unsigned)A.G.deg[root];
             if (threadIdx.x == 0) {
@@ -612,6 +653,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                 qd[0] = root;
                 lvl[0] = 0;
                 sm.tail = 1;
+                sm.next = sm.nbig = 0;
+                sm.slots[1] = sm.long_slots[1] = 0;
                 sm.lvslots[0] = front;
                 sm.lvlong[0] = (int)front >= push_deg() ? front + (1ull << kLongShift) : 0ull;
                 V[root >> 5] |= 1u << (root & 31);
@@ -620,19 +663,17 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
             // ---- forward: levels 0, 1, ... ----
             int L = 0, lo = 0, hi = 1;
             bool held = false;  // kOneBits: B is a copy of V
+            __syncthreads();
             for (;;) {
-                const unsigned long long rest = total - visited;
+                const unsigned long long rest = sm.total - visited;
                 // the scan for unvisited vertices itself costs about a slot per four vertices
                 const bool pull = sym && rest + (unsigned long long)(nv >> 2) < front;
                 // a level that may have more vertices than the bitmap has words
                 // is listed from N when it is complete, in vertex order
                 const bool dense = pull || front >= (unsigned)nw;
                 uint32_t* const N = pull ? Npull : Npush;
-                if (threadIdx.x == 0) sm.next = sm.nbig = 0;
-                __syncthreads();
-                if (threadIdx.x == 0) sm.slots = sm.long_slots = 0;
                 if (!pull) {
-                    scanned += front;
+                    if (threadIdx.x == 0) sm.scanned += front;
                     const uint32_t* T = MODE == kOneBits ? B : V;
                     if (MODE == kOneBits && !held) {
                         for (int i = threadIdx.x; i < nw; i += NT) B[i] = V[i];
@@ -642,10 +683,11 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                     // An unvisited neighbour gains x's sigma and joins N; where
                     // the level is short its first visitor, the one that sets
                     // the bit, also lists it.
-                    auto act = [&](long long s, const int (&k)[kLaneSlots]) {
+                    auto act = [&](long long s, const auto& k) {
+                        constexpr int S = std::extent<std::remove_reference_t<decltype(k)>>::value;
                         const unsigned in = present(k) & ~in_bitmap(T, k);
 #pragma unroll
-                        for (int u = 0; u < kLaneSlots; ++u)
+                        for (int u = 0; u < S; ++u)
                             if ((in >> u) & 1u) {
                                 if (MODE == kSmall) add_shared(&Sg[k[u]], s);
                                 else atomic_add_i64(&Sg[k[u]], s);
@@ -653,17 +695,17 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                         unsigned first = in & ~in_bitmap(N, k);
                         if (dense) {
 #pragma unroll
-                            for (int u = 0; u < kLaneSlots; ++u)
+                            for (int u = 0; u < S; ++u)
                                 if ((first >> u) & 1u) atomicOr(&N[k[u] >> 5], 1u << (k[u] & 31));
                             return;
                         }
                         if (first) {
-                            unsigned old[kLaneSlots];
+                            unsigned old[S];
 #pragma unroll
-                            for (int u = 0; u < kLaneSlots; ++u)
+                            for (int u = 0; u < S; ++u)
                                 old[u] = (first >> u) & 1u ? atomicOr(&N[k[u] >> 5], 1u << (k[u] & 31)) : ~0u;
 #pragma unroll
-                            for (int u = 0; u < kLaneSlots; ++u) {
+                            for (int u = 0; u < S; ++u) {
                                 if ((old[u] >> (k[u] & 31)) & 1u) first &= ~(1u << u);
                                 if ((first >> u) & 1u) D[k[u]] = L + 1;
                             }
@@ -671,7 +713,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                         append_first(sm, qd, k, first);
                     };
                     list_tasks<NT, long long>(A.G, sm, qd + lo, hi - lo, front, [&](int x) { return (long long)Sg[x]; },
-                                              [&](const TaskVertex<long long>& q, bool) { push_batch(A.G, sm, q, act); });
+                                              [&](const TaskVertex<long long>& q, bool) { push_batch<kFew>(A.G, sm, q, act); });
                     big_segments(A.G, sm, [&](int, int x, int64_t rs, int s0, int s1) {
                         const long long s = Sg[x];
                         for (int i = s0 + lane; i < s1; i += 32 * kLaneSlots) {
@@ -682,7 +724,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                         __syncwarp();
                     });
                 } else {
-                    scanned += rest;
+                    if (threadIdx.x == 0) sm.scanned += rest;
                     if (MODE == kOneBits && held) {
                         for (int i = threadIdx.x; i < nw; i += NT) B[i] = 0u;
                         held = false;
@@ -695,7 +737,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                         if (hit) atomicOr(&N[x >> 5], 1u << (x & 31));
                     };
                     unset_tasks<NT>(A.G, sm, V, nw, [&](const TaskVertex<int>& q, bool ok) {
-                        pull_batch<int64_t>(A.G, sm, q, ok, B, Sg, done);
+                        pull_batch<kFew, int64_t>(A.G, sm, q, ok, B, Sg, done);
                     });
                     const int nb = big_segments(A.G, sm, [&](int b, int x, int64_t rs, int s0, int s1) {
                         int64_t s = 0;
@@ -715,12 +757,17 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                         }
                     });
                     if (nb > 0) {
-                        __syncthreads();
                         for (int b = threadIdx.x; b < nb; b += NT)
                             done(sm.big[b], Sg[sm.big[b]], sm.bighit[b] != 0);
+                        __syncthreads();
                     }
                 }
-                __syncthreads();
+                // every thread has read the level's counts; the other buffer
+                // holds the next level's
+                if (threadIdx.x == 0) {
+                    sm.next = sm.nbig = 0;
+                    sm.slots[L & 1] = sm.long_slots[L & 1] = 0;
+                }
                 // B and N are empty again between levels (or B is the visited set)
                 if (pull)
                     for (int i = lo + threadIdx.x; i < hi; i += NT) B[qd[i] >> 5] = 0u;
@@ -728,7 +775,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                 auto count = [&](int x) {
                     const unsigned d = (unsigned)A.G.deg[x];
                     sum += d;
-                    if ((int)d >= push_deg()) longs += d + (1ull << kLongShift);
+                    if (d >= kPushDegMin && (int)d >= push_deg()) longs += d + (1ull << kLongShift);
                 };
                 lo = hi;
                 if (dense) {
@@ -778,21 +825,23 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                 }
                 if (lo == hi) break;
                 ++L;
+                if (__any_sync(full, sum != 0)) {
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(full, sum, o);
-                if (lane == 0 && sum) atomicAdd(&sm.slots, sum);
-                if (__any_sync(full, longs != 0)) {
+                    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(full, sum, o);
+                    if (lane == 0) atomicAdd(&sm.slots[L & 1], sum);
+                    if (__any_sync(full, longs != 0)) {
 #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) longs += __shfl_xor_sync(full, longs, o);
-                    if (lane == 0) atomicAdd(&sm.long_slots, longs);
+                        for (int o = 16; o > 0; o >>= 1) longs += __shfl_xor_sync(full, longs, o);
+                        if (lane == 0) atomicAdd(&sm.long_slots[L & 1], longs);
+                    }
                 }
                 if (threadIdx.x == 0) lvl[L] = lo;
                 __syncthreads();
-                front = sm.slots;
+                front = sm.slots[L & 1];
                 visited += front;
                 if (threadIdx.x == 0 && L < kSlotLevels) {
                     sm.lvslots[L] = front;
-                    sm.lvlong[L] = sm.long_slots;
+                    sm.lvlong[L] = sm.long_slots[L & 1];
                 }
             }
             nlev = L + 1;
@@ -837,7 +886,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                                                     q.d = 0;
                                                     ok = false;
                                                 }
-                                                pull_batch<double>(A.G, sm, q, ok, B, acc,
+                                                pull_batch<kFew, double>(A.G, sm, q, ok, B, acc,
                                                                    [&](int y, double sum, bool) { finish(y, sum); });
                                             });
                     const int nb = big_segments(A.G, sm, [&](int, int x, int64_t rs, int s0, int s1) {
@@ -855,10 +904,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                         }
                     });
                     if (nb > 0) {
-                        __syncthreads();
                         for (int b = threadIdx.x; b < nb; b += NT) finish(sm.big[b], acc[sm.big[b]]);
+                        __syncthreads();
                     }
-                    __syncthreads();
                     for (int i = a1 + threadIdx.x; i < end; i += NT) B[qd[i] >> 5] = 0u;
                     if (threadIdx.x == 0) sm.next = sm.nbig = 0;
                     __syncthreads();
@@ -870,14 +918,15 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                     }
                     if (threadIdx.x == 0) sm.scanned += sm.lvslots[l + 1];
                     __syncthreads();
-                    auto act = [&](double w, const int (&k)[kLaneSlots]) {
+                    auto act = [&](double w, const auto& k) {
+                        constexpr int S = std::extent<std::remove_reference_t<decltype(k)>>::value;
                         const unsigned in = in_bitmap(B, k);
 #pragma unroll
-                        for (int u = 0; u < kLaneSlots; ++u)
+                        for (int u = 0; u < S; ++u)
                             if ((in >> u) & 1u) atomicAdd(&acc[k[u]], w);
                     };
                     list_tasks<NT, double>(A.G, sm, qd + a1, end - a1, sm.lvslots[l + 1], [&](int x) { return acc[x]; },
-                                           [&](const TaskVertex<double>& q, bool) { push_batch(A.G, sm, q, act); });
+                                           [&](const TaskVertex<double>& q, bool) { push_batch<kFew>(A.G, sm, q, act); });
                     big_segments(A.G, sm, [&](int, int x, int64_t rs, int s0, int s1) {
                         const double w = acc[x];
                         for (int i = s0 + lane; i < s1; i += 32 * kLaneSlots) {
@@ -887,7 +936,6 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                         }
                         __syncwarp();
                     });
-                    __syncthreads();
                     for (int i = a0 + threadIdx.x; i < a1; i += NT) {
                         const int x = qd[i];
                         if (bit_of(B, x)) finish(x, acc[x]);
@@ -963,7 +1011,6 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
             // the reference counts every reached vertex and its degree in both passes
             sm.walked_v += 2ull * (unsigned)reached;
             sm.walked_e += 2ull * visited;
-            sm.scanned += scanned;
         }
         __syncthreads();
     }
