@@ -548,6 +548,11 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
     const int lane = threadIdx.x & 31;
     const int64_t nv = A.nv;
     const int nw = (int)((nv + 31) / 32);
+    const unsigned nx = (unsigned)nw * 32;  // vertices, up to whole words
+    // vertices per thread of a pass over all of them, loads first: with few
+    // roots a pass is a chain of load latencies (a 2 M vertex graph, an isolated
+    // root 1.97 -> 1.56 ms, 152 roots 3.68 -> 2.58)
+    constexpr int kUnroll = MODE == kSmall ? 1 : 4;
     constexpr bool kFew = MODE != kSmall;
     const bool sym = !A.asym && !(A.asym_dev && *A.asym_dev);
 
@@ -623,18 +628,23 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
         {
             unsigned long long sum = 0;
             int most = 0;
-            for (int64_t x = threadIdx.x; x < (int64_t)nw * 32; x += NT) {
-                int d = 0;
-                if (x < nv) {
-                    d = A.G.deg[x];
-                    D[x] = SBC_INF;
-                    Sg[x] = 0;
-                    if (MODE == kSmall) acc[x] = 0.0;
+            for (unsigned x0 = threadIdx.x; x0 < nx; x0 += kUnroll * NT) {
+                int d[kUnroll];
+#pragma unroll
+                for (int u = 0; u < kUnroll; ++u) d[u] = x0 + u * NT < nv ? A.G.deg[x0 + u * NT] : 0;
+#pragma unroll
+                for (int u = 0; u < kUnroll; ++u) {
+                    const unsigned x = x0 + u * NT;
+                    if (x < nv) {
+                        D[x] = SBC_INF;
+                        Sg[x] = 0;
+                        if (MODE == kSmall) acc[x] = 0.0;
+                    }
+                    sum += (unsigned)d[u];
+                    most = max(most, d[u]);
+                    const unsigned word = __ballot_sync(full, x >= nv || (sym && d[u] == 0));
+                    if (lane == 0 && x < nx) V[x >> 5] = word;
                 }
-                sum += (unsigned)d;
-                most = max(most, d);
-                const unsigned word = __ballot_sync(full, x >= nv || (sym && d == 0));
-                if (lane == 0) V[x >> 5] = word;
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(full, sum, o);
@@ -951,40 +961,50 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
 
         // ---- the rows, and what is derived from the levels ----
         uint32_t* D2 = A.dist2 ? A.dist2 + (size_t)r * d2_words(nv) : nullptr;
-        for (int64_t x = threadIdx.x; x < (int64_t)nw * 32; x += NT) {
-            const int d = x < nv ? D[x] : SBC_INF;
-            if (x < nv) {
-                D8[x] = enc_d8(d);
-                if (MODE == kSmall) {
-                    gD[x] = d;
-                    gS[x] = Sg[x];
-                } else if (d != SBC_INF) {
-                    acc[x] = 0.0;
-                }
-                if (d == SBC_INF) Dl[x] = 0.0;
-            }
-            if (D2) {
-                // two bits per vertex: the ballots of the low and the high
-                // bits, spread to even and odd places
-                const unsigned c = enc_d2(d);
-                unsigned even = __ballot_sync(full, c & 1u), odd = __ballot_sync(full, c & 2u);
-                if (lane < 2) {
-                    if (lane) {
-                        even >>= 16;
-                        odd >>= 16;
+        for (unsigned x0 = threadIdx.x; x0 < nx; x0 += kUnroll * NT) {
+            int d[kUnroll];
+            unsigned even[kUnroll], odd[kUnroll];
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) d[u] = x0 + u * NT < nv ? D[x0 + u * NT] : SBC_INF;
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) {
+                const unsigned x = x0 + u * NT;
+                if (x < nv) {
+                    D8[x] = enc_d8(d[u]);
+                    if (MODE == kSmall) {
+                        gD[x] = d[u];
+                        gS[x] = Sg[x];
+                    } else if (d[u] != SBC_INF) {
+                        acc[x] = 0.0;
                     }
-                    auto spread = [](unsigned v) {
-                        v &= 0xffffu;
-                        v = (v | (v << 8)) & 0x00ff00ffu;
-                        v = (v | (v << 4)) & 0x0f0f0f0fu;
-                        v = (v | (v << 2)) & 0x33333333u;
-                        return (v | (v << 1)) & 0x55555555u;
-                    };
-                    const int64_t word = ((x - lane) >> 4) + lane;
-                    if (word < d2_words(nv)) D2[word] = spread(even) | (spread(odd) << 1);
+                    if (d[u] == SBC_INF) Dl[x] = 0.0;
                 }
+                const unsigned c = enc_d2(d[u]);
+                even[u] = __ballot_sync(full, c & 1u);
+                odd[u] = __ballot_sync(full, c & 2u);
+                if (MODE >= kOneBits && lane == 0 && x < nx) V[x >> 5] = 0u;
             }
-            if (MODE >= kOneBits && lane == 0) V[x >> 5] = 0u;
+            // two bits per vertex: the ballots of the low and the high bits,
+            // spread to even and odd places, half a ballot a lane
+            if (D2 && lane < 2 * kUnroll) {
+                unsigned e = even[0], o = odd[0];
+#pragma unroll
+                for (int u = 1; u < kUnroll; ++u)
+                    if (lane >> 1 == u) {
+                        e = even[u];
+                        o = odd[u];
+                    }
+                auto spread = [](unsigned v) {
+                    v &= 0xffffu;
+                    v = (v | (v << 8)) & 0x00ff00ffu;
+                    v = (v | (v << 4)) & 0x0f0f0f0fu;
+                    v = (v | (v << 2)) & 0x33333333u;
+                    return (v | (v << 1)) & 0x55555555u;
+                };
+                const int half = lane & 1;
+                const int64_t word = ((int64_t)(x0 - lane + (lane >> 1) * NT) >> 4) + half;
+                if (word < d2_words(nv)) D2[word] = spread(e >> (16 * half)) | (spread(o >> (16 * half)) << 1);
+            }
         }
         if (A.hist) {
             for (int t = threadIdx.x; t < kHistLevels; t += NT) {
