@@ -164,17 +164,17 @@ cudaError_t build_adjacency(int64_t nv, const int64_t* off, const int64_t* adj, 
         }
     }
     auto cleanup = [&]() {
-        for (void* p : {(void*)d_off, (void*)d_adj, (void*)d_tmp_off, (void*)d_short, (void*)d_long, (void*)d_tmp,
-                        (void*)d_skew})
+        for (void* p : {(void*)d_off, (void*)d_adj, (void*)d_tmp_off, (void*)d_short, (void*)d_long, (void*)d_tmp})
             if (p) cudaFree(p);
     };
-    if ((e = cudaMalloc(&d_off, sizeof(int64_t) * (nv + 1))) ||
+    // the skew's word follows the offsets
+    if ((e = cudaMalloc(&d_off, sizeof(int64_t) * (nv + 2))) ||
         (e = cudaMalloc(&d_adj, sizeof(int64_t) * std::max<int64_t>(ne, 1))) ||
         (e = cudaMalloc(&d_short, sizeof(int32_t) * std::max<size_t>(shortl.size(), 1))) ||
         (e = cudaMalloc(&d_long, sizeof(int32_t) * std::max<size_t>(longl.size(), 1))) ||
         (e = cudaMalloc(&d_tmp_off, sizeof(int64_t) * std::max<size_t>(tmp_off.size(), 1))) ||
         (e = cudaMalloc(&d_tmp, sizeof(int32_t) * std::max<int64_t>(tmp_total, 1))) ||
-        (e = cudaMalloc(&d_skew, sizeof *d_skew)) || (e = cudaMemsetAsync(d_skew, 0, sizeof *d_skew, s)) ||
+        (e = cudaMemsetAsync(d_skew = (unsigned long long*)d_off + nv + 1, 0, sizeof *d_skew, s)) ||
         (e = cudaMemcpyAsync(d_off, off, sizeof(int64_t) * (nv + 1), cudaMemcpyHostToDevice, s)) ||
         (ne && (e = cudaMemcpyAsync(d_adj, adj, sizeof(int64_t) * ne, cudaMemcpyHostToDevice, s))) ||
         (!shortl.empty() &&
