@@ -847,6 +847,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                 }
                 if (threadIdx.x == 0) lvl[L] = lo;
                 __syncthreads();
+                // the slots of parents whose level the way up cannot look up
+                if (threadIdx.x == 0 && L >= kSlotLevels) sm.scanned += front;
                 front = sm.slots[L & 1];
                 visited += front;
                 if (threadIdx.x == 0 && L < kSlotLevels) {

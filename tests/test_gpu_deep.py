@@ -61,3 +61,18 @@ def test_deep_and_short_levels(sbc_lib, port_lib, name):
     o.close()
     f.close()
     dg.close()
+
+
+@pytest.mark.parametrize("nv", [40, 63, 64, 65, 66, 67, 300, 9000])
+def test_scanned_slots_of_a_path(sbc_lib, nv):
+    """From one end of a path every level is one vertex: all slots are read on the way down, and on the way up those
+    of every vertex but the last, or one fewer where the last two levels are walked from the last."""
+    g = G.from_edges(nv, np.arange(nv - 1), np.arange(1, nv))
+    dg = native.DeviceGraph(g.nv, g.off, g.adj)
+    f = native.DeviceForest(dg, [0])
+    f.counters()
+    f.static_init()
+    down = 2 * (nv - 1)
+    assert down + down - 2 <= f.counters()["scanned"] <= down + down - 1
+    f.close()
+    dg.close()
