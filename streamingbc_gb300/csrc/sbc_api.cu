@@ -79,12 +79,20 @@ int ensure_staging(sbc_graph* g, int64_t n)
     if (n <= g->ins_capacity) return SBC_OK;
     int cap = (int)std::max<int64_t>(n, 64);
     CK(cudaStreamSynchronize(g->stream));  // queued batches may still read the old staging
+    // the old one stays until both parts of the new one are there: every call
+    // on the graph reads its results through it
+    int32_t *d = nullptr, *h = nullptr;
+    cudaError_t e;
+    if ((e = dev_alloc(&d, (size_t)5 * cap + 1)) ||  // u, v, codes, two rank rows and a flag (launch_append)
+        (e = cudaMallocHost((void**)&h, sizeof(int32_t) * (4 * (size_t)cap + kCallResultInts)))) {
+        dev_free(d);
+        cudaGetLastError();  // reported here, not by the next launch
+        return cuda_fail(e, "batch staging allocation");
+    }
     if (g->d_ins) cudaFree(g->d_ins);
     if (g->h_ins) cudaFreeHost(g->h_ins);
-    g->d_ins = nullptr;
-    g->h_ins = nullptr;
-    CK(dev_alloc(&g->d_ins, (size_t)5 * cap + 1));  // u, v, codes, two rank rows and a flag (launch_append)
-    CK(cudaMallocHost((void**)&g->h_ins, sizeof(int32_t) * (4 * (size_t)cap + kCallResultInts)));
+    g->d_ins = d;
+    g->h_ins = h;
     g->ins_capacity = cap;
     return SBC_OK;
 }
