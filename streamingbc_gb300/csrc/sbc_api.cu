@@ -200,10 +200,17 @@ int stage_host(sbc_graph* g, int64_t n, const int64_t* u, const int64_t* v, bool
             hv[i] = -1;
         }
     }
-    // the rows in one copy
-    const size_t pitch = sizeof(int32_t) * (size_t)cap;
-    CK(cudaMemcpy2DAsync(g->d_ins, pitch, hu, pitch, sizeof(int32_t) * (size_t)n, set_ok ? 3 : 2, cudaMemcpyHostToDevice,
-                         g->stream));
+    // the rows in one copy, or one each where they are further apart than a
+    // pitched copy allows (2 GB)
+    const size_t pitch = sizeof(int32_t) * (size_t)cap, width = sizeof(int32_t) * (size_t)n;
+    const int rows = set_ok ? 3 : 2;
+    if (pitch < (size_t)1 << 31) {
+        CK(cudaMemcpy2DAsync(g->d_ins, pitch, hu, pitch, width, rows, cudaMemcpyHostToDevice, g->stream));
+    } else {
+        for (int i = 0; i < rows; ++i)
+            CK(cudaMemcpyAsync(g->d_ins + (size_t)i * cap, hu + (size_t)i * cap, width, cudaMemcpyHostToDevice,
+                               g->stream));
+    }
     CK(cudaEventRecord(g->staged, g->stream));
     return SBC_OK;
 }
