@@ -1254,6 +1254,24 @@ int sbc_graph_remove_directed(sbc_graph* g, int64_t from, int64_t to, int* resul
     return SBC_OK;
 }
 
+namespace {
+// The recompute of a deletion's roots could not be carried out (no memory for
+// it, say).  Their dependencies have left BC already, so the forest has no
+// valid state any more: updates are refused until the next static init.
+int recompute_failed(sbc_forest* f, cudaError_t e, const char* where)
+{
+    cudaStream_t s = f->g->stream;
+    cudaGetLastError();  // reported here, not by the next launch
+    f->initialized = false;
+    cudaMemsetAsync(f->d_dcnt, 0, sizeof(int), s);
+    cudaMemsetAsync(f->d_dirty, 0, sizeof(int) * (size_t)f->nk, s);
+    f->ws.clear(s);
+    const int rc = cuda_fail(e, where);
+    t_err += " (the forest needs sbc_static_init)";
+    return rc;
+}
+}  // namespace
+
 int sbc_delete_batch(sbc_forest* f, int64_t n, const int64_t* u, const int64_t* v, sbc_batch_stats* stats)
 {
     if (f && !f->g) return fail(SBC_ERR_STATE, "sbc_delete_batch: the forest's graph was destroyed");
@@ -1290,7 +1308,8 @@ int sbc_delete_batch(sbc_forest* f, int64_t n, const int64_t* u, const int64_t* 
         }
     if (stats) fill_stats(g, n, R->counters, stats);
     if (R->dirty > 0) {
-        CK(sbc::launch_delete_finish(f, R->dirty));
+        const cudaError_t e = sbc::launch_delete_finish(f, R->dirty);
+        if (e) return recompute_failed(f, e, "sbc_delete_batch recompute");
         if (stats) {  // the recomputes count as traversals
             CK(cudaMemcpyAsync(R->counters, f->d_counters, sizeof R->counters, cudaMemcpyDeviceToHost, g->stream));
             CK(cudaMemsetAsync(f->d_counters, 0, sizeof R->counters, g->stream));
@@ -1318,7 +1337,8 @@ int sbc_update_deleted(sbc_forest* f, int64_t u, int64_t v, sbc_batch_stats* sta
     static const int kRemoved = 1;
     CK(cudaMemcpyAsync(g->d_err + 1, &kRemoved, sizeof(int), cudaMemcpyHostToDevice, g->stream));
     if (stats) CK(cudaMemsetAsync(f->d_counters, 0, sizeof(unsigned long long) * SBC_NCOUNTERS, g->stream));
-    CK(sbc::launch_delete(f, (int)u, (int)v, g->d_err + 1));
+    const cudaError_t e = sbc::launch_delete(f, (int)u, (int)v, g->d_err + 1);
+    if (e) return recompute_failed(f, e, "sbc_update_deleted");
     CallResult* R = g->h_result();
     if (stats) {
         CK(cudaMemcpyAsync(R->counters, f->d_counters, sizeof R->counters, cudaMemcpyDeviceToHost, g->stream));

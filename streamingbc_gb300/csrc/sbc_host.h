@@ -97,6 +97,12 @@ struct WorkerScratch {
         }
         workers = w;
         nv = n;
+        return clear(s);
+    }
+    cudaError_t clear(cudaStream_t s)
+    {
+        const size_t sc = (size_t)workers * (size_t)nv, words = (size_t)workers * sbc::bitmap_words(nv);
+        cudaError_t e;
         if ((e = cudaMemsetAsync(st, 0, sc * 4, s)) || (e = cudaMemsetAsync(dp, 0, sc * 8, s)) ||
             (e = cudaMemsetAsync(acc, 0, sc * 8, s)) || (e = cudaMemsetAsync(bits, 0, words * 4, s)))
             return e;
