@@ -601,14 +601,18 @@ __device__ __forceinline__ void lb_walk_sum(const DevGraph& G, int g, const Dist
     }
 }
 
-// Child weights (delta + 1) / sigma.  An SM issues one fp64 instruction per 16
+// Child weights (delta + 1) / sigma.  An SM issues one fp64 instruction per 20
 // cycles, each waiting for the one before, and the compiler's division is the
 // longest chain of them in a commit.  Here the reciprocal of sigma starts from
 // the fp32 one (24 bits), one Newton step doubles its bits, and the quotient's
-// remainder, exact by fused multiply-add, corrects the quotient to the last bit
-// (Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", 1990): five fp64 instructions, three where the reciprocal is at
-// hand.
+// remainder corrects the quotient (after Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990): five fp64
+// instructions, three where the reciprocal is at hand.  The quotient before the
+// correction is good to some 45 bits, so its remainder, one fused multiply-add,
+// is itself rounded; what is left of both errors is below 2^-39 of the last
+// place before the final rounding, so a result differs from the division's by
+// one unit in the last place at most, and only where the exact quotient lies
+// that close to the middle of two doubles.
 struct Sigma {
     double b, r;  // its value and its reciprocal to about 46 bits (0: divide plainly)
 };
