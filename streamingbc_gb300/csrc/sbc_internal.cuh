@@ -400,9 +400,10 @@ __device__ __forceinline__ void gather_dist(const DistRow& dr, const int (&kk)[I
 // walk_fetch, a warp reading one contiguous run; the distance is gathered from
 // the root's one-byte row D8, falling back to the int32 row D only for levels
 // >= 254).  post(j, x) runs after the chunk's edges.  Ends with a barrier.
-// REF: the walked vertices and their degrees count as traversed in the
-// reference's sense (COUNT_TRAVERSALS); every walk counts its scanned slots.
-template <int NT, bool REF = true, int ILP = kEdgeIlp, bool TOMB = false, class Prep, class Edge, class Post>
+// Every walk counts its scanned slots; those of lb_walk_ahead also count the
+// walked vertices and their degrees as traversed in the reference's sense
+// (COUNT_TRAVERSALS).
+template <int NT, int ILP = kEdgeIlp, bool TOMB = false, class Prep, class Edge, class Post>
 __device__ __forceinline__ void lb_walk(const DevGraph& G, int g, const DistRow dr,
                                         const int32_t* l1, int n1, const int32_t* l2, int n2, LbSmem<NT>& sm,
                                         Prep prep, Edge edge, Post post)
@@ -426,10 +427,6 @@ __device__ __forceinline__ void lb_walk(const DevGraph& G, int g, const DistRow 
         if (t < cnt) sm.off[t] = off;
         if (t == 0) {
             sm.off[cnt] = total;
-            if (REF) {
-                sm.walked_v += (unsigned)cnt;
-                sm.walked_e += (unsigned)total;
-            }
             sm.scanned_e += (unsigned)total;
         }
         __syncthreads();

@@ -38,8 +38,6 @@ __device__ __forceinline__ void flag_rebuild(int32_t* flag, int32_t* list, int32
     if (atomicExch(&flag[r], 1) == 0) list[atomicAdd(cnt, 1)] = r;
 }
 
-constexpr int kL1Warps = 1;
-
 // Builds the masks of root r (one CTA).  Every slot of the root and of its
 // neighbours is an edge (called between batches: deg0 == deg).
 __device__ __forceinline__ void build_root(DevGraph G, const int64_t* roots, uint32_t* mask, int32_t* cand,
@@ -58,15 +56,15 @@ __device__ __forceinline__ void build_root(DevGraph G, const int64_t* roots, uin
     const int64_t rr = G.row[root];
     for (int i = threadIdx.x; i < rdeg; i += blockDim.x) C[i] = G.col[rr + i];
     __syncthreads();
-    // kL1Warps warps per neighbour, so that all lists are read at once: one list
+    // a warp per neighbour, so that all lists are read at once: one list
     // after the other by the whole CTA was a chain of up to 32 list starts (ER
     // 1,024, 1,024 roots: 23 us)
-    const int team = threadIdx.x / (32 * kL1Warps), lane = threadIdx.x % (32 * kL1Warps);
-    for (int i = team; i < rdeg; i += blockDim.x / (32 * kL1Warps)) {
+    const int lane = threadIdx.x & 31;
+    for (int i = threadIdx.x >> 5; i < rdeg; i += blockDim.x >> 5) {
         const int y = C[i];
         const int64_t ry = G.row[y];
         const int dy = G.deg[y];
-        for (int s = lane; s < dy; s += 32 * kL1Warps) atomicOr(&M[G.col[ry + s]], 1u << i);
+        for (int s = lane; s < dy; s += 32) atomicOr(&M[G.col[ry + s]], 1u << i);
     }
     if (threadIdx.x == 0) l1n[r] = rdeg;
 }

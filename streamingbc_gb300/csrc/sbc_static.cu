@@ -1155,8 +1155,7 @@ size_t static_fixed(int nt, int mode)
 StaticKernel static_kernel(int nt, int mode)
 {
     if (mode == kSmall)
-        return nt == 128 ? k_static<128, kSmall> : nt == 256 ? k_static<256, kSmall>
-             : nt == 512 ? k_static<512, kSmall> : k_static<1024, kSmall>;
+        return nt == 128 ? k_static<128, kSmall> : nt == 256 ? k_static<256, kSmall> : k_static<512, kSmall>;
     if (mode == kBits)
         return nt <= 256 ? k_static<256, kBits> : nt == 512 ? k_static<512, kBits> : k_static<1024, kBits>;
     return mode == kOneBits ? k_static<1024, kOneBits> : k_static<1024, kNoBits>;
@@ -1321,8 +1320,8 @@ __global__ void k_csr_degrees(const int64_t* __restrict__ off, int64_t nv, int32
 // Input check on the device, before k_static touches anything: a root outside
 // [0, nv), an offset array that does not start at 0 or decreases, or a
 // neighbour id outside [0, nv) sets a bit of *bad (1 roots, 2 offsets, 4
-// neighbour ids).  k_static and k_bc_colsum_checked read the word and do
-// nothing when it is set, so a bad id never becomes an out-of-bounds access.
+// neighbour ids).  k_static and k_bc_colsum read the word and do nothing when
+// it is set, so a bad id never becomes an out-of-bounds access.
 // The neighbour ids read are d_col[0 .. d_off[nv]), the caller's CSR.
 __global__ void k_noalloc_check(const int64_t* __restrict__ off, const int32_t* __restrict__ col, int64_t nv,
                                 const int64_t* __restrict__ roots, int64_t nk, int* __restrict__ bad)

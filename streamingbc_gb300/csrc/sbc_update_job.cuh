@@ -512,7 +512,7 @@ __device__ __forceinline__ void ascend(const ForestSlot& A, UpdSmem<NT>& sm, con
                         pull_walk(A.G.col + rrow, rdeg);
                     } else {
                         const int nscan = sm.nscan, nprobe = sm.nprobe;
-                        lb_walk<NT, false, ILP, TOMB>(A.G, g, DistRow{D, D8, D2, L}, W.qs + qbase, nscan, nullptr, 0, sm.lb,
+                        lb_walk<NT, ILP, TOMB>(A.G, g, DistRow{D, D8, D2, L}, W.qs + qbase, nscan, nullptr, 0, sm.lb,
                                                 prep_loaded,
                                            [&](int j, int x, int k, int dk) { parent_edge(j, x, k, dk, kNoAux); },
                                                 NoPost());
@@ -679,7 +679,7 @@ __device__ bool movedown(const ForestSlot& A, UpdSmem<NT>& sm, const Scratch& W,
     bool over = false;
     while (lo < hi) {
         const int c_lo = sm.at;
-        lb_walk<NT, false, ILP, TOMB>(A.G, g, row, W.qs + lo, hi - lo, nullptr, 0, sm.lb, noprep,
+        lb_walk<NT, ILP, TOMB>(A.G, g, row, W.qs + lo, hi - lo, nullptr, 0, sm.lb, noprep,
                                 [&](int, int, int k, int dk) {
                                     if (dk != l + 1 || W.st[k] != 0) return;
                                     const int old = atomicCAS(&W.st[k], 0, kDecCand);
@@ -687,7 +687,7 @@ __device__ bool movedown(const ForestSlot& A, UpdSmem<NT>& sm, const Scratch& W,
                                 },
                                 NoPost());
         const int c_hi = sm.at;
-        lb_walk<NT, false, ILP, TOMB>(A.G, g, row, W.qa + c_lo, c_hi - c_lo, nullptr, 0, sm.lb, noprep,
+        lb_walk<NT, ILP, TOMB>(A.G, g, row, W.qa + c_lo, c_hi - c_lo, nullptr, 0, sm.lb, noprep,
                                 [&](int, int k, int y, int dy) {
                                     if (dy != l) return;
                                     if (W.st[y] & kDecAff) atomic_add_i64(&W.dp[k], S[y]);
@@ -733,7 +733,7 @@ __device__ bool movedown(const ForestSlot& A, UpdSmem<NT>& sm, const Scratch& W,
     // ---- 2. new levels of X (held in the step bits; SBC_STEP_MASK = none) ----
     for (int i = threadIdx.x; i < nx; i += NT) W.st[W.qs[i]] = kDecAff | SBC_STEP_MASK;
     __syncthreads();
-    lb_walk<NT, false, ILP, TOMB>(A.G, g, row, W.qs, nx, nullptr, 0, sm.lb, noprep,
+    lb_walk<NT, ILP, TOMB>(A.G, g, row, W.qs, nx, nullptr, 0, sm.lb, noprep,
                             [&](int, int x, int y, int dy) {
                                 if (dy == SBC_INF || (W.st[y] & kDecAff)) return;
                                 const int want = kDecAff | (dy + 1);
@@ -753,7 +753,7 @@ __device__ bool movedown(const ForestSlot& A, UpdSmem<NT>& sm, const Scratch& W,
             warp_append(&sm.qt, W.qd, x, (W.st[x] & SBC_STEP_MASK) == L);
         }
         __syncthreads();
-        lb_walk<NT, false, ILP, TOMB>(A.G, g, row, W.qd, sm.qt, nullptr, 0, sm.lb, noprep,
+        lb_walk<NT, ILP, TOMB>(A.G, g, row, W.qd, sm.qt, nullptr, 0, sm.lb, noprep,
                                 [&](int, int, int z, int) {
                                     const int sz = W.st[z];
                                     if ((sz & kDecAff) && (sz & SBC_STEP_MASK) > L + 1)
@@ -810,7 +810,7 @@ __device__ bool movedown(const ForestSlot& A, UpdSmem<NT>& sm, const Scratch& W,
         const int seg_lo = W.lvl[step];
         if (threadIdx.x == 0) W.lvl[step + 1] = end;
         // X vertices of this level: sigma from the new parents one level up
-        lb_walk<NT, false, ILP, TOMB>(A.G, g, row, W.qd + p_hi, x_hi - p_hi, nullptr, 0, sm.lb, noprep,
+        lb_walk<NT, ILP, TOMB>(A.G, g, row, W.qd + p_hi, x_hi - p_hi, nullptr, 0, sm.lb, noprep,
                                 [&](int, int x, int y, int dy) {
                                     const int sy = W.st[y];
                                     int ly;
@@ -829,7 +829,7 @@ __device__ bool movedown(const ForestSlot& A, UpdSmem<NT>& sm, const Scratch& W,
                                 NoPost());
         // unaffected vertices of this level: their sigma changes to their
         // unaffected children (never to an X vertex)
-        lb_walk<NT, false, ILP, TOMB>(
+        lb_walk<NT, ILP, TOMB>(
             A.G, g, row, W.qd + seg_lo, p_hi - seg_lo, W.qd + x_hi, end - x_hi, sm.lb,
             [&](int j, int x, int) { sm.dp[j] = W.dp[x]; },
             [&](int j, int, int k, int dk) {
