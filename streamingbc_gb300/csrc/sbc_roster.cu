@@ -10,11 +10,13 @@
 // parents of such a vertex by binary search for each roster member in its
 // sorted adjacency (same parents, same results).
 //
-// Levels only shrink under insertions, and a vertex only moves to a shallower
-// level (in a re-levelling descent), which appends it to its new level's
-// roster; its old entry is left in place and marked stale.  Rosters are
-// therefore supersets of their levels, readers check distances, and
-// k_roster_compact drops stale entries after each batch.
+// Under insertions a vertex only moves to a shallower level (in a re-levelling
+// descent), under deletions only to a deeper one (a move-down); it is appended
+// to its new level's roster, and its old entry is left in place and marked
+// stale.  Within a call no vertex comes back to a level that it left, so
+// rosters are supersets of their levels that name no vertex twice (a reader
+// adds a parent's share once per entry); readers check distances, and
+// k_roster_compact drops stale entries after each call that moves vertices.
 //   k_roster_build    CTA per root: members of levels 2..kRosterLevels-1 whose
 //                     level histogram count fits a roster (after static init)
 //   k_roster_compact  thread per (root, level) roster, the warp together for

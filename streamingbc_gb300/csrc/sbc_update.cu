@@ -394,6 +394,7 @@ cudaError_t launch_delete_step(sbc_forest* f, int u, int v, const int* d_removed
     A.counters = f->d_counters;
     k_delete<512, 1, 4><<<(int)std::min<int64_t>(f->workers, f->nk), 512, 0, s>>>(A);
     if ((e = cudaGetLastError())) return e;
+    if (md && (e = launch_roster_compact(f, s))) return e;
     // the others: their dependencies out of BC now (their state is still that
     // of the graph before this deletion), recomputed at the end of the batch
     const dim3 grid((unsigned)std::min<int64_t>((f->nv + 255) / 256, 64), (unsigned)std::min<int64_t>(f->nk, 4096));
@@ -490,7 +491,10 @@ cudaError_t launch_delete_batch(sbc_forest* f, int n)
             break;
         }
     shape->launch(A, (int)std::min<int64_t>(f->workers, f->nk), s);
-    return cudaGetLastError();
+    if ((e = cudaGetLastError())) return e;
+    // before a later insertion brings a vertex that moved down back to a level
+    // whose roster still lists it
+    return A.move_down ? launch_roster_compact(f, s) : cudaSuccess;
 }
 
 cudaError_t launch_delete(sbc_forest* f, int u, int v, const int* d_removed)
