@@ -25,6 +25,7 @@ def _start(nv, seed):
     def device(pairs):
         d = torch.tensor(np.asarray(pairs), dtype=torch.int32, device="cuda")
         u, v = d[:, 0].contiguous(), d[:, 1].contiguous()
+        torch.cuda.synchronize()  # they are made on another stream than the forest's
         f.insert_device(len(d), u.data_ptr(), v.data_ptr())
         f.sync()
 
