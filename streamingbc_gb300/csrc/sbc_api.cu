@@ -693,14 +693,17 @@ int sbc_graph_create(sbc_graph** out, int64_t nv, const int64_t* off, const int6
         sbc_graph_destroy(g);
         return cuda_fail(e, "sbc_graph_create allocation");
     }
-    if ((e = cudaMemcpy(g->d_row, g->h_row.data(), sizeof(int64_t) * (nv + 1), cudaMemcpyHostToDevice)) ||
-        (nv && (e = cudaMemcpy(g->d_deg, deg.data(), sizeof(int32_t) * nv, cudaMemcpyHostToDevice))) ||
-        (nv && (e = cudaMemcpy(g->d_deg0, deg.data(), sizeof(int32_t) * nv, cudaMemcpyHostToDevice))) ||
-        (nv && (e = cudaMemcpy(g->d_nsort, deg.data(), sizeof(int32_t) * nv, cudaMemcpyHostToDevice))) ||
-        (nv && (e = cudaMemcpy(g->d_cap, g->h_cap.data(), sizeof(int32_t) * nv, cudaMemcpyHostToDevice))) ||
-        (e = cudaMemset(g->d_col, 0, sizeof(int32_t) * std::max<int64_t>(total, 1))) ||
-        (e = cudaMemset(g->d_seq, 0, sizeof(int32_t) * std::max<int64_t>(total, 1))) ||
-        (e = cudaMemset(g->d_err, 0, 2 * sizeof(int)))) {
+    // on the graph's own stream, which takes no notice of the default one:
+    // a copy or fill left there may come after the build below
+    const cudaStream_t s = g->stream;
+    if ((e = cudaMemcpyAsync(g->d_row, g->h_row.data(), sizeof(int64_t) * (nv + 1), cudaMemcpyHostToDevice, s)) ||
+        (nv && (e = cudaMemcpyAsync(g->d_deg, deg.data(), sizeof(int32_t) * nv, cudaMemcpyHostToDevice, s))) ||
+        (nv && (e = cudaMemcpyAsync(g->d_deg0, deg.data(), sizeof(int32_t) * nv, cudaMemcpyHostToDevice, s))) ||
+        (nv && (e = cudaMemcpyAsync(g->d_nsort, deg.data(), sizeof(int32_t) * nv, cudaMemcpyHostToDevice, s))) ||
+        (nv && (e = cudaMemcpyAsync(g->d_cap, g->h_cap.data(), sizeof(int32_t) * nv, cudaMemcpyHostToDevice, s))) ||
+        (e = cudaMemsetAsync(g->d_col, 0, sizeof(int32_t) * std::max<int64_t>(total, 1), s)) ||
+        (e = cudaMemsetAsync(g->d_seq, 0, sizeof(int32_t) * std::max<int64_t>(total, 1), s)) ||
+        (e = cudaMemsetAsync(g->d_err, 0, 2 * sizeof(int), s))) {
         sbc_graph_destroy(g);
         return cuda_fail(e, "sbc_graph_create upload");
     }
@@ -1379,7 +1382,7 @@ int sbc_cost_log_start(sbc_forest* f, int64_t capacity)
         if ((e = dev_alloc(&M->d_x, (size_t)capacity * sbc::kIn)) || (e = dev_alloc(&M->d_y, (size_t)capacity)))
             return cuda_fail(e, "cost log allocation");
         M->capacity = capacity;
-        CK(cudaMemset(M->d_n, 0, sizeof(unsigned long long)));
+        CK(cudaMemsetAsync(M->d_n, 0, sizeof(unsigned long long), f->g->stream));
     }
     M->logging = true;
     drop_captured(f);
@@ -1587,7 +1590,9 @@ int sbc_cost_model_params(sbc_forest* f, float* get, const float* set)
     if (rc) return rc;
     CK(cudaStreamSynchronize(f->g->stream));
     if (set) {
-        CK(cudaMemcpy(f->model->d_params, set, sizeof(float) * sbc::kModelParams, cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(f->model->d_params, set, sizeof(float) * sbc::kModelParams, cudaMemcpyHostToDevice,
+                           f->g->stream));
+        CK(cudaStreamSynchronize(f->g->stream));
         f->model->trained = true;
         drop_captured(f);
     }
@@ -1604,7 +1609,7 @@ int sbc_cost_model_predict(sbc_forest* f, int64_t n, const float* x, float* out)
     float *dx = nullptr, *dout = nullptr;
     cudaError_t e;
     if ((e = dev_alloc(&dx, (size_t)n * sbc::kIn)) || (e = dev_alloc(&dout, (size_t)n)) ||
-        (e = cudaMemcpy(dx, x, sizeof(float) * n * sbc::kIn, cudaMemcpyHostToDevice)) ||
+        (e = cudaMemcpyAsync(dx, x, sizeof(float) * n * sbc::kIn, cudaMemcpyHostToDevice, f->g->stream)) ||
         (e = sbc::launch_predict(f->model->d_params, dx, n, dout, f->g->stream)) ||
         (e = cudaStreamSynchronize(f->g->stream)) ||
         (e = cudaMemcpy(out, dout, sizeof(float) * n, cudaMemcpyDeviceToHost))) {
@@ -1627,8 +1632,8 @@ int sbc_cost_model_grad(sbc_forest* f, int64_t n, const float* x, const float* y
     cudaStream_t s = f->g->stream;
     if ((e = dev_alloc(&dx, (size_t)n * sbc::kIn)) || (e = dev_alloc(&dy, (size_t)n)) ||
         (e = dev_alloc(&dg, (size_t)sbc::kTrainParams)) || (e = dev_alloc(&dp, (size_t)n)) ||
-        (e = cudaMemcpy(dx, x, sizeof(float) * n * sbc::kIn, cudaMemcpyHostToDevice)) ||
-        (e = cudaMemcpy(dy, y, sizeof(float) * n, cudaMemcpyHostToDevice)) ||
+        (e = cudaMemcpyAsync(dx, x, sizeof(float) * n * sbc::kIn, cudaMemcpyHostToDevice, s)) ||
+        (e = cudaMemcpyAsync(dy, y, sizeof(float) * n, cudaMemcpyHostToDevice, s)) ||
         (e = cudaMemsetAsync(dg, 0, sizeof(float) * sbc::kTrainParams, s)) ||
         (e = sbc::launch_grad(f->model->d_params, dg, dx, dy, 0, n, n, 1, 0, dp, s)) ||
         (e = cudaStreamSynchronize(s)) ||

@@ -42,3 +42,29 @@ def test_static_init_beside_other_graphs(sbc_lib, port_lib, sizes, reps):
     for d, f in zip(dgs, fs):
         f.close()
         d.close()
+
+
+def test_graphs_built_beside_work_on_the_default_stream(sbc_lib):
+    """A graph's arrays are filled on its own stream, whatever another thread has queued on the default one."""
+    torch = pytest.importorskip("torch")
+    g = G.er(3000, 30000, seed=1)
+    x = torch.randn(2048, 2048, device="cuda")
+    stop = threading.Event()
+
+    def busy():
+        while not stop.is_set():
+            for _ in range(20):
+                torch.mm(x, x)
+            torch.cuda.default_stream().synchronize()
+
+    t = threading.Thread(target=busy)
+    t.start()
+    try:
+        for _ in range(60):
+            dg = native.DeviceGraph(g.nv, g.off, g.adj)
+            off, adj = dg.to_csr()
+            dg.close()
+            assert (off == g.off).all() and (adj == g.adj).all()
+    finally:
+        stop.set()
+        t.join()
