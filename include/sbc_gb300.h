@@ -377,7 +377,9 @@ int sbc_forest_set_delete_mode(sbc_forest *f, int mode);
  * each, as n single deletions would.  One update launch serves the whole
  * call: the removed slots stay marked in place until it ends, so each
  * deletion's jobs see the graph without the edges of that deletion and the
- * earlier ones.  Synchronous; stats may be NULL. */
+ * earlier ones.  Synchronous; stats may be NULL.  If a recompute cannot be
+ * carried out (no memory, say) the call fails and the forest refuses updates
+ * until sbc_static_init. */
 int sbc_delete_batch(sbc_forest *f, int64_t n, const int64_t *u, const int64_t *v, sbc_batch_stats *stats);
 /* The update for one deletion whose edge the caller has already removed in
  * both directions (sbc_graph_remove_directed x2, or stinger_remove_edge x2),

@@ -1,6 +1,6 @@
 """Static init where its kernel changes form: the working set of a root in
 shared memory, only the bitmaps there, one of them or none (by vertex count),
-vertices scanned by a thread, eight lanes, a warp or the CTA (by degree), levels
+vertices scanned by a thread, 4 or 16 lanes, a warp or the CTA (by degree), levels
 walked from above or below, and adjacencies that are not symmetric.  dist and
 sigma bit-exact against the oracle, BC within the 1e-9 of the parity tests."""
 import numpy as np
