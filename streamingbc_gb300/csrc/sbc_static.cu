@@ -65,8 +65,9 @@ constexpr int kSlotLevels = 64;   // levels whose slot counts the backward pass 
 // kBigDeg, and beyond in segments of kSegSlots that the CTA's warps share out.
 // A task none of whose vertices has more than kFewSlots takes a shorter form of
 // the one-lane step: deep graphs are bound by the instructions of the few warps
-// that have work (a path of 20,000, one root 69.8 -> 59.4 ms; where whole rows
-// are in shared memory the test cost ER 1,024 as much as it gave paths).
+// that have work (a path of 20,000, one root 69.8 -> 59.4 ms).  Not where whole
+// rows are in shared memory: the graphs that live there have such tasks on
+// their outermost levels alone (ER 1,024 would lose half a percent).
 constexpr int kLaneSlots = 8, kFewSlots = 4;
 constexpr int kBigDeg = 1024;
 constexpr int kSegSlots = 2048;
@@ -79,10 +80,10 @@ constexpr int kSegSlots = 2048;
 //   R-MAT 20, 8              2.9e-15 | 4.4e-14 | 2.6e-15
 //   Chung-Lu 40k, 64         9.2e-16 | 1.3e-15 | 6.8e-16
 //   5 hubs, 100k leaves, 16  1.4e-14 | 1.9e-12 | 9.5e-16
-// Without the lower bound Chung-Lu (degrees to 300) would scan a third more
-// slots; 1/8 puts R-MAT 18 at 4.1e-15.  The time of the two last forms: R-MAT
-// 18, 251 roots 9.4 | 10.7 ms, R-MAT 20, 304 roots 44.4 | 46.3 ms, Chung-Lu
-// 40k, 256 roots 1.15 | 1.22 ms; a star of 5,000, 300 roots 1.41 | 0.18 ms.
+// 1/8 puts R-MAT 18 at 4.1e-15, a lower bound of 256 Chung-Lu 40k at 1.4e-15.
+// The time of the two last forms: R-MAT 18, 251 roots 9.4 | 10.7 ms, R-MAT 20,
+// 304 roots 44.4 | 46.3 ms, Chung-Lu 40k, 256 roots 1.15 | 1.22 ms (1.30 with a
+// lower bound of 64); a star of 5,000, 300 roots 1.41 | 0.18 ms.
 constexpr int kPushDegMin = 128, kPushDegMax = 4096, kPushDegPart = 16;
 constexpr int kLongShift = 40;
 // Vertices of kBigDeg or more listed per walk (the others stay a warp's).

@@ -218,7 +218,7 @@ constexpr int kDefaultVariant = 7;  // 1024 threads, one root per SM
 //                           K=256  2915 |  2538 |  2519 |  2972 |  3430
 //                           K=500  3495 |  3091 |  3733 |  4606 |  5459
 //   ER 1024, 16 k           K=1024 2343 |  2571 |  3735 |     - |  6023
-//   R-MAT 14, 222 k         K=152  3413 |  2416 |  1982 |  1851 |  1951
+//   R-MAT 14, 228 k         K=152  3413 |  2416 |  1982 |  1851 |  1951
 //                           K=500  5278 |  3778 |  3065 |  3286 |  3582
 //   Chung-Lu 40k, 352 k     K=152 10142 |  6362 |  4626 |  4387 |  4167
 //                           K=256  9070 |  5836 |  4410 |  5395 |  5659
@@ -229,7 +229,7 @@ constexpr int kDefaultVariant = 7;  // 1024 threads, one root per SM
 //   Chung-Lu 100k, 1.2 M    K=152 11229 |  6765 |  4701 |  4438 |  4085
 //                           K=256 22302 | 12732 |  8124 |  8285 |  6793
 //                           K=500 23276 | 13473 |  9318 | 10234 |  9592
-//   R-MAT 17, 3.6 M         K=152 20394 | 10672 |  6225 |  5868 |  4562
+//   R-MAT 17, 3.7 M         K=152 20394 | 10672 |  6225 |  5868 |  4562
 //                           K=500 61992 | 31869 | 18096 | 17786 | 13276
 // Small graphs are bound by the latency of a job's steps, so as many roots in
 // flight as there are, and a CTA no narrower than they need; from about 0.5 M
