@@ -848,8 +848,6 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
                 }
                 if (threadIdx.x == 0) lvl[L] = lo;
                 __syncthreads();
-                // the slots of parents whose level the way up cannot look up
-                if (threadIdx.x == 0 && L >= kSlotLevels) sm.scanned += front;
                 front = sm.slots[L & 1];
                 visited += front;
                 if (threadIdx.x == 0 && L < kSlotLevels) {
@@ -872,6 +870,14 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_static(const __grid_constant_
             };
             for (int i = lvl[nlev - 1] + threadIdx.x; i < reached; i += NT) finish(qd[i], 0.0);
             if (threadIdx.x == 0) sm.next = sm.nbig = 0;
+            if (nlev > kSlotLevels) {
+                // parents below the counted levels are all pulled: the slots of
+                // every vertex but those of the counted levels and the last one
+                for (int i = lvl[nlev - 1] + threadIdx.x; i < reached; i += NT)
+                    atomicAdd(&sm.scanned, 0ull - (unsigned)A.G.deg[qd[i]]);
+                if (threadIdx.x < kSlotLevels - 1) atomicAdd(&sm.scanned, 0ull - sm.lvslots[threadIdx.x]);
+                if (threadIdx.x == 0) atomicAdd(&sm.scanned, visited);
+            }
             __syncthreads();
             int end = reached;  // of level l + 1
             for (int l = nlev - 2; l >= 0; --l) {
