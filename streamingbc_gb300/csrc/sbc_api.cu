@@ -665,7 +665,6 @@ int sbc_graph_create(sbc_graph** out, int64_t nv, const int64_t* off, const int6
     g->h_row.resize(nv + 1);
     g->h_cap.resize(nv);
     g->h_deg_ub.resize(nv);
-    g->h_freed.assign(nv, 0);
     std::vector<int32_t> deg(nv);
     int64_t total = 0;
     for (int64_t v = 0; v < nv; ++v) {
@@ -1252,7 +1251,7 @@ int sbc_graph_remove_directed(sbc_graph* g, int64_t from, int64_t to, int* resul
     CK(cudaStreamSynchronize(g->stream));
     if (*result == 1) {
         g->edge_skew -= sbc::edge_mix((int)from, (int)to);
-        g->h_freed[from]++;
+        g->slot_freed(from);
     }
     return SBC_OK;
 }
@@ -1306,8 +1305,8 @@ int sbc_delete_batch(sbc_forest* f, int64_t n, const int64_t* u, const int64_t* 
     const int32_t* codes = g->h_codes();
     for (int64_t i = 0; i < n; ++i)
         if (codes[i] > 0) {
-            g->h_freed[u[i]]++;
-            g->h_freed[v[i]]++;
+            g->slot_freed(u[i]);
+            g->slot_freed(v[i]);
         }
     if (stats) fill_stats(g, n, R->counters, stats);
     if (R->dirty > 0) {

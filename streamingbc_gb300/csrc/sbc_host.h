@@ -156,10 +156,15 @@ struct sbc_graph {
     // was reserved for: the slack also takes batches that were not, and those
     // are in no bound until the next planned batch reads the degrees.
     std::vector<int64_t> h_deg_ub;
-    std::vector<int64_t> h_freed;
+    std::vector<int64_t> h_freed;  // empty until the first removal
     int64_t reserved = 0;     // pairs reserved that no device batch has used yet
     bool unreserved = false;  // a device batch went beyond what was reserved since the degrees were read
-    int64_t deg_bound(int64_t v) const { return h_deg_ub[v] - (unreserved ? 0 : h_freed[v]); }
+    int64_t deg_bound(int64_t v) const { return h_deg_ub[v] - (unreserved || h_freed.empty() ? 0 : h_freed[v]); }
+    void slot_freed(int64_t v)
+    {
+        if (h_freed.empty()) h_freed.assign(nv, 0);
+        h_freed[v]++;
+    }
     // staging for insertion batches
     int ins_capacity = 0;
     int32_t* d_ins = nullptr;  // [5 * ins_capacity + 1]: u, v, ok, then the append's ranks and misfit flag
